@@ -92,6 +92,247 @@ gemm_rows_kernel(const TX* __restrict__ X, const TW* __restrict__ W, const void*
     }
 }
 
+// ---- float32 operands in 16-byte pieces (K and the row stride of X multiples of 4, aligned bases): the 32-bit path itself.
+// Products are taken two at a time by fma.rn.f32x2 (two independent float32 FMAs with the usual rounding), the pair being two
+// neighbouring k: both operands then lie in shared memory as they lie in global memory (no transposition), and a sum is kept as
+// an even-k and an odd-k half that are added at the end.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ float halves_sum(f32x2 v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ float bias_at(const void* bias, int bias_dtype, int n) {
+    return bias_dtype == LLB_F32 ? ((const float*)bias)[n] : to_f32(((const bf16*)bias)[n]);
+}
+
+// Up to eight rows: bound by streaming W.  A warp takes four weight rows; the block's eight warps are 8 / wk groups of
+// four rows times wk shares of K (interleaved 512-byte pieces), added in shared memory in a fixed order.  UNROLL pieces of four
+// rows, 4 * UNROLL loads of 16 bytes a lane, are requested before the first is used.  (One warp a row with 4-byte loads, one in
+// flight, before: 93 us a product on average in a one-token step of the 28-layer 1.5B shape, 0.6 TB/s.  Now 5.3 TB/s for one row
+// against 151,936 x 1,536 and 4.1 for eight, 3.7 and 2.2 against 1,536 x 8,960; the step 11.4 -> 2.1 ms.)
+template <int MR, int UNROLL>
+__global__ void __launch_bounds__(256, 2)
+gemm_rows_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const void* __restrict__ bias, int bias_dtype,
+                     float* __restrict__ Y, int M, int N, int K, int ldx, int ldy, int wk) {
+    constexpr int R = 4, NV = R * MR;
+    __shared__ float red[8][NV];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int share = warp % wk, group = warp / wk, groups = 8 / wk;
+    const int n0 = (blockIdx.x * groups + group) * R;
+    const float* w[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = W + (size_t)min(n0 + r, N - 1) * K;
+    const float* x[MR];
+#pragma unroll
+    for (int i = 0; i < MR; ++i) x[i] = X + (size_t)min(i, M - 1) * ldx;
+    float acc[R][MR];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < MR; ++i) acc[r][i] = 0.f;
+    llb_grid_dependency_sync();
+    const int step = wk * 128;
+    int k = (share * 32 + lane) * 4;
+    auto take = [&](const float4* wv, int at) {
+#pragma unroll
+        for (int i = 0; i < MR; ++i) {
+            const float4 xv = *reinterpret_cast<const float4*>(x[i] + at);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                acc[r][i] = fmaf(xv.w, wv[r].w, fmaf(xv.z, wv[r].z, fmaf(xv.y, wv[r].y, fmaf(xv.x, wv[r].x, acc[r][i]))));
+        }
+    };
+    for (; k + (UNROLL - 1) * step < K; k += UNROLL * step) {
+        float4 wv[UNROLL][R];
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u)
+#pragma unroll
+            for (int r = 0; r < R; ++r) wv[u][r] = __ldcs(reinterpret_cast<const float4*>(w[r] + k + u * step));
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) take(wv[u], k + u * step);
+    }
+    for (; k < K; k += step) {
+        float4 wv[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) wv[r] = __ldcs(reinterpret_cast<const float4*>(w[r] + k));
+        take(wv, k);
+    }
+    // the warp's sums: at every step a lane keeps one half of the values and hands the other half to its partner
+    float v[NV];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < MR; ++i) v[r * MR + i] = acc[r][i];
+#pragma unroll
+    for (int n = NV, o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool upper = lane & o;
+#pragma unroll
+            for (int j = 0; j < NV / 2; ++j)
+                if (j < n) {
+                    const float give = upper ? v[j] : v[j + n], keep = upper ? v[j + n] : v[j];
+                    v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    constexpr int COPIES = 32 / NV;              // lanes that hold the same value; value lane / COPIES = r * MR + i
+    if (lane % COPIES == 0) red[warp][lane / COPIES] = v[0];
+    __syncthreads();
+    if (threadIdx.x < groups * NV) {
+        const int g = threadIdx.x / NV, at = threadIdx.x - g * NV, i = at / R, r = at - i * R;     // neighbours: a row's columns
+        const int n = (blockIdx.x * groups + g) * R + r;
+        if (i < M && n < N) {
+            float s = 0.f;
+            for (int q = 0; q < wk; ++q) s += red[g * wk + q][r * MR + i];
+            Y[(size_t)i * ldy + n] = bias ? s + bias_at(bias, bias_dtype, n) : s;
+        }
+    }
+}
+
+// More rows: bound by the FMA units.  A block computes ROWS x 128 outputs from a ring of three k-blocks of 32 (cp.async, 16-byte
+// pieces, rows 144 bytes apart so that eight neighbouring rows are read without bank conflicts); a thread has TM x 8
+// outputs (16 TM FMAs for every TM + 8 loads of 16 bytes).  With ROWS = 64, two blocks of four warps share an SM; rows of 16
+// and 32 are for products that would leave most of a tile empty (41 and 56 us for 16 and 32 rows against 17,920 x 1,536, 95 with 64).
+// At 46 TFLOP/s (256 x 151,936 x 1,536) shared-memory reads, a byte an FMA, take as long as the FMAs.  (4-byte loads, a
+// transposing store and 4 x 4 outputs a thread before: 13 TFLOP/s; a 256-token step of the 1.5B shape 59 -> 24 ms.)
+// gridDim.z > 1: K is cut into ranges, each range's partial product goes to its plane of `part`, and gemm_planes_f32_kernel adds them.
+constexpr int F_BN = 128, F_BK = 32, F_PITCH = F_BK + 4, F_STAGES = 3;
+template <int ROWS, int TM>
+__global__ void __launch_bounds__(ROWS / TM * 16, ROWS >= 64 ? 2 : 3)
+gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const void* __restrict__ bias, int bias_dtype,
+                float* __restrict__ Y, float* __restrict__ part, int M, int N, int K, int ldx, int ldy, int m_tiles, int k_range) {
+    constexpr int THREADS = ROWS / TM * 16, TN = 8;
+    constexpr int STAGE = (ROWS + F_BN) * F_PITCH;                     // floats
+    extern __shared__ __align__(16) float ring[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = (blockIdx.x % m_tiles) * ROWS, n0 = (blockIdx.x / m_tiles) * F_BN;
+    const int k_lo = blockIdx.z * k_range, k_hi = min(K, k_lo + k_range), n_blocks = (k_hi - k_lo + F_BK - 1) / F_BK;
+    llb_grid_dependency_sync();
+
+    auto fetch = [&](int kb) {
+        float* st = ring + (kb % F_STAGES) * STAGE;
+        const int k0 = k_lo + kb * F_BK;
+#pragma unroll
+        for (int i = tid; i < (ROWS + F_BN) * (F_BK / 4); i += THREADS) {
+            const int row = i / (F_BK / 4), k = k0 + (i % (F_BK / 4)) * 4;
+            const bool is_x = row < ROWS;
+            const int at = is_x ? m0 + row : n0 + row - ROWS;
+            const bool in = k < k_hi && at < (is_x ? M : N);
+            const float* src = in ? (is_x ? X + (size_t)at * ldx : W + (size_t)at * K) + k : X;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(st + row * F_PITCH + (i % (F_BK / 4)) * 4);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+        }
+    };
+    // a warp's outputs: 4 TM rows x 64 columns; lane (ly, lx) has rows ly + 4 i and columns lx + 8 j of them
+    const int lx = lane & 7, ly = lane >> 3, wn = warp & 1, wm = warp >> 1;
+    f32x2 acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+#pragma unroll
+    for (int s = 0; s < F_STAGES - 1; ++s) {
+        if (s < n_blocks) fetch(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int kb = 0; kb < n_blocks; ++kb) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(F_STAGES - 2) : "memory");
+        __syncthreads();                         // block kb is there for all; all have finished the block whose place is filled next
+        if (kb + F_STAGES - 1 < n_blocks) fetch(kb + F_STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* xs = ring + (kb % F_STAGES) * STAGE + (wm * 4 * TM + ly) * F_PITCH;
+        const float* ws = ring + (kb % F_STAGES) * STAGE + (ROWS + wn * 64 + lx) * F_PITCH;
+#pragma unroll
+        for (int k = 0; k < F_BK; k += 4) {
+            ulonglong2 b[TN];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 8 * F_PITCH + k);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + i * 4 * F_PITCH + k);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.x, b[j].x);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.y, b[j].y);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const bool planes = gridDim.z > 1;
+    float* out = planes ? part + (size_t)blockIdx.z * M * N : Y;
+    const int ldo = planes ? N : ldy;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + wm * 4 * TM + ly + 4 * i;
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + wn * 64 + lx + 8 * j;
+            if (n >= N) continue;
+            float v = halves_sum(acc[i][j]);
+            if (bias && !planes) v += bias_at(bias, bias_dtype, n);
+            out[(size_t)m * ldo + n] = v;
+        }
+    }
+}
+
+// Y = sum of the planes, in their order, + bias
+__global__ void __launch_bounds__(256)
+gemm_planes_f32_kernel(const float* __restrict__ part, int planes, const void* __restrict__ bias, int bias_dtype, float* __restrict__ Y,
+                       int M, int N, int ldy) {
+    llb_grid_dependency_sync();
+    const size_t n_all = (size_t)M * N;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n_all; i += (size_t)gridDim.x * 256) {
+        float s = part[i];
+        for (int q = 1; q < planes; ++q) s += part[q * n_all + i];
+        const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
+        Y[(size_t)m * ldy + n] = bias ? s + bias_at(bias, bias_dtype, n) : s;
+    }
+}
+
+// Rows of a tile: the smallest that holds M, 64 beyond 32.
+static int f32_tile_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
+
+// K ranges of the product of more than eight rows: as many as make the rounds of blocks times the k-blocks of a range smallest;
+// a round's set-up counts as two k-blocks, a plane that is written and read again as one.
+static int f32_splits(int M, int N, int K, int sms) {
+    const int rows = f32_tile_rows(M), blocks = (K + F_BK - 1) / F_BK;
+    const long long tiles = (long long)((M + rows - 1) / rows) * ((N + F_BN - 1) / F_BN), room = (long long)sms * (rows >= 64 ? 2 : 3);
+    int best = 1;
+    long long best_cost = -1;
+    for (int s = 1; s <= 16 && s * 4 <= blocks; ++s) {
+        const int range = (blocks + s - 1) / s;
+        if ((long long)range * (s - 1) >= blocks) continue;           // the last range would be empty
+        const long long cost = (tiles * s + room - 1) / room * (range + 2) + (s > 1 ? 4 + s : 0);
+        if (best_cost < 0 || cost < best_cost) { best = s; best_cost = cost; }
+    }
+    return best;
+}
+
+template <int ROWS, int TM>
+static int launch_f32(const float* X, const float* W, const void* bias, int bias_dtype, float* Y, float* part, int M, int N, int K,
+                      int ldx, int ldy, int splits, cudaStream_t stream) {
+    auto kernel = gemm_f32_kernel<ROWS, TM>;
+    constexpr int SMEM = F_STAGES * (ROWS + F_BN) * F_PITCH * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return -2000 - (int)e;
+    const int m_tiles = (M + ROWS - 1) / ROWS, blocks = (K + F_BK - 1) / F_BK;
+    const long long tiles = (long long)m_tiles * ((N + F_BN - 1) / F_BN);
+    if (tiles > 2147483647ll) return (int)cudaErrorInvalidValue;
+    llb_launch(kernel, dim3((unsigned)tiles, 1, splits), dim3(ROWS / TM * 16), SMEM, stream, X, W, bias, bias_dtype, Y, part, M, N, K, ldx,
+               ldy, m_tiles, (blocks + splits - 1) / splits * F_BK);
+    if (splits > 1)
+        llb_launch(gemm_planes_f32_kernel, dim3((unsigned)min(((size_t)M * N + 255) / 256, (size_t)148 * 16)), dim3(256), 0, stream,
+                   (const float*)part, splits, bias, bias_dtype, Y, M, N, ldy);
+    return llb_status();
+}
+
+static bool f32_pieces(const void* X, int x_dtype, const void* W, int w_dtype, int y_dtype, int K, int ldx) {
+    return x_dtype == LLB_F32 && w_dtype == LLB_F32 && y_dtype == LLB_F32 && K > 0 && K % 4 == 0 && ldx % 4 == 0 &&
+           (((uintptr_t)X | (uintptr_t)W) & 15) == 0;
+}
+
 template <typename TX, typename TW, typename TO>
 static void launch(const void* X, const void* W, const void* bias, int bias_dtype, void* Y, int M,
                    int N, int K, int ldx, int ldy, cudaStream_t stream) {
@@ -107,11 +348,38 @@ static void launch(const void* X, const void* W, const void* bias, int bias_dtyp
     }
 }
 
-// ldx, ldy: row strides of X and Y in elements (W is dense [N, K]).
+// Float32 elements of scratch that llb_gemm_simt wants for these operands (0: none): the planes of a K that is cut into ranges.
+LLB_API long long llb_gemm_simt_scratch(const void* X, int x_dtype, const void* W, int w_dtype, int y_dtype, int M, int N, int K,
+                                        int ldx, int sms) {
+    if (M <= 8 || N <= 0 || !f32_pieces(X, x_dtype, W, w_dtype, y_dtype, K, ldx)) return 0;
+    const int s = f32_splits(M, N, K, sms);
+    return s > 1 ? (long long)s * M * N : 0;
+}
+
+// ldx, ldy: row strides of X and Y in elements (W is dense [N, K]).  part: scratch of `part_elems` float32 (may be null with 0);
+// K is cut into as many ranges as it holds planes of M x N.
 LLB_API int llb_gemm_simt(const void* X, int x_dtype, const void* W, int w_dtype, const void* bias,
                           int bias_dtype, void* Y, int y_dtype, int M, int N, int K, int ldx,
-                          int ldy, cudaStream_t stream) {
+                          int ldy, float* part, long long part_elems, int sms, cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
+    if (f32_pieces(X, x_dtype, W, w_dtype, y_dtype, K, ldx)) {
+        const float *x = (const float*)X, *w = (const float*)W;
+        if (M <= 8) {
+            // shares of K: until the grid has four blocks for every SM, while a lane keeps two pieces
+            int wk = 1;
+            while (wk < 8 && (long long)(N + 31) / 32 * wk < 4ll * sms && K >= wk * 2 * 256) wk *= 2;
+            const dim3 grid((N + 32 / wk - 1) / (32 / wk));
+            auto kernel = M == 1 ? gemm_rows_f32_kernel<1, 4> : M == 2 ? gemm_rows_f32_kernel<2, 2>
+                        : M <= 4 ? gemm_rows_f32_kernel<4, 2> : gemm_rows_f32_kernel<8, 2>;
+            llb_launch(kernel, grid, dim3(256), 0, stream, x, w, bias, bias_dtype, (float*)Y, M, N, K, ldx, ldy, wk);
+            return llb_status();
+        }
+        int splits = f32_splits(M, N, K, sms);
+        if (!part || part_elems < (long long)splits * M * N) splits = 1;
+        return M <= 16 ? launch_f32<16, 2>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream)
+             : M <= 32 ? launch_f32<32, 4>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream)
+                       : launch_f32<64, 8>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream);
+    }
     if ((N + 63) / 64 > 2147483647 || (M + 63) / 64 > 65535) return (int)cudaErrorInvalidValue;
     LLB_DISPATCH_DTYPE(x_dtype, TX, {
         LLB_DISPATCH_DTYPE(w_dtype, TW, {

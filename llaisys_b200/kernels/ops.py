@@ -107,11 +107,11 @@ def _check(rc: int, what: str, n: int = 1):
 _configured = set()
 
 
-def _fn(lib, name, argtypes):
+def _fn(lib, name, argtypes, restype=c_int):
     f = getattr(lib, name)
     if (id(lib), name) not in _configured:
         f.argtypes = argtypes
-        f.restype = c_int
+        f.restype = restype
         _configured.add((id(lib), name))
     return f
 
@@ -604,11 +604,19 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if _tc_ok(x, weight, bias) and (out.is_contiguous() or (out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0 and N % 8 == 0)):
         _gemm_tc(x, weight, bias, out, plan=plan)
         return out
-    lib = load_module("gemm_simt.cu")
+    lib, sms, part = load_module("gemm_simt.cu"), _sm_count(x.device), None
+    if M > 8 and K >= 256 and x.dtype == torch.float32:
+        # few tiles: K is cut into ranges whose partial products lie in planes of scratch (up to eight rows, or a K of fewer
+        # than eight k-blocks, need none)
+        f = _fn(lib, "llb_gemm_simt_scratch", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int], c_longlong)
+        elems = f(_ptr(x), _dt(x), _ptr(weight), _dt(weight), _dt(out), M, N, K, x.stride(0), sms)
+        if elems:
+            part = torch.empty((elems,), dtype=torch.float32, device=x.device)
     f = _fn(lib, "llb_gemm_simt", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int,
-                                   c_int, c_int, c_int, c_int, c_int, c_void_p])
+                                   c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p])
     _check(f(_ptr(x), _dt(x), _ptr(weight), _dt(weight), _ptr(bias), _dt(bias) if bias is not None else 0,
-             _ptr(out), _dt(out), M, N, K, x.stride(0), out.stride(0), _stream()), "linear")
+             _ptr(out), _dt(out), M, N, K, x.stride(0), out.stride(0), _ptr(part), 0 if part is None else part.numel(), sms, _stream()),
+           "linear", 1 if part is None else 2)
     return out
 
 

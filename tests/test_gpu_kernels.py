@@ -101,6 +101,25 @@ def test_linear(dtype, M, N, K):
     assert np.abs(got.double().cpu().numpy() - want).max() < 1e-4 * math.sqrt(K)
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 16, 17, 32, 33, 64, 65, 200])
+@pytest.mark.parametrize("N,K,pad", [(1, 4, 0), (127, 36, 4), (130, 1028, 0), (520, 2048, 12), (33, 8960, 0)])
+def test_linear_f32_in_pieces(M, N, K, pad):
+    """The 32-bit product in 16-byte pieces: every row count at which another kernel or tile takes over, ragged tiles, K ranges
+    that are cut and that end inside a k-block, a row stride; and an input whose base is off the 16 bytes.  A float32 sum of K
+    products in any order differs from the exact one by at most K 2^-24 times the sum of their magnitudes; here 8 times
+    sqrt(K) instead of K (roundings do not all fall the same way)."""
+    from llaisys_b200 import kernels
+    gen = torch.Generator(device=DEV).manual_seed(M * 1000 + N + K)
+    buf = torch.randn(M * (K + pad) + 4, device=DEV, generator=gen)
+    w, b = torch.randn(N, K, device=DEV, generator=gen), torch.randn(N, device=DEV, generator=gen)
+    for off, bias in ((0, b), (0, None), (1, b.to(torch.bfloat16))):
+        x = buf[off:off + M * (K + pad)].view(M, K + pad)[:, :K]
+        want = x.double() @ w.double().T + (0 if bias is None else bias.double())
+        size = x.double().abs() @ w.double().abs().T + (0 if bias is None else bias.double().abs())
+        got = kernels.linear(x, w, bias)
+        assert bool(((got.double() - want).abs() <= 2.0 ** -24 * max(8.0, math.sqrt(K)) * size).all())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_swiglu(dtype):
     from llaisys_b200 import kernels
