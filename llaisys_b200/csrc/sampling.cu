@@ -161,153 +161,331 @@ LLB_API int llb_argmax_split(const float* logits, long long ld, int R, int V, in
     return llb_status();
 }
 
-// exclusive prefix sum over the block's threads; total returned through *total
-__device__ unsigned long long block_excl_scan(unsigned long long v, unsigned long long* sh,
-                                              unsigned long long* total) {
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// ---- sampling: a row belongs to a cluster of eight blocks, each of which keeps its eighth of the row in shared memory
+//
+// The rule needs a dozen passes over a row (the maximum, three digits of the k-th largest key, the kept mass, three digits of the
+// nucleus' cut, the draw).  With one block per row they all came from the L2 at one SM's rate: 571 us for 64 rows of 151,936, whose one
+// read from memory takes 6 (now 110).  Here the row is read once, the passes run over shared memory, and the blocks exchange what they
+// must (histograms of a digit, sums) through each other's shared memory between cluster barriers.  Every sum is one of
+// integers, so how a row is divided does not change the result.
+constexpr int ST = 512, SWARPS = ST / 32, SC = 8;         // threads of a block, blocks of a row
+constexpr int BINS = 2048, SLICE = BINS / SC;             // values of a digit; a block adds up its slice of them over the cluster
+constexpr int SMEM_MAX = 232448;
+
+struct SampleShared {
+    // a digit's histogram over this block's elements: counts and masses.  The masses (at most 2^40 each) are added in parts of 14,
+    // 14 and 13 bits while 2^18 elements a block are out of reach, because 64-bit atomics on shared memory are loops
+    uint32_t cnt[BINS];
+    union { uint32_t mass[3][BINS]; unsigned long long whole_mass[BINS]; };
+    unsigned long long scan[SWARPS + 1];
+    // written by the cluster's blocks, read behind a cluster barrier
+    ArgMax peer_max[SC];
+    uint32_t peer_warp_max[SC * SWARPS];
+    unsigned long long peer_sum[4][SC];
+    unsigned long long peer_cnt[SC], peer_mass[SC];
+    uint32_t digit, above;                                // the chosen digit, and how many elements lie above it
+    unsigned long long acc;                               // ... and their mass
+    // the block's own
+    ArgMax red[SWARPS];
+    uint32_t floor_key, lowest;
+};
+
+__device__ __forceinline__ unsigned long long mass_fp(float logit, float mx, float inv_t) {
+    float e = expf((logit - mx) * inv_t);
+    if (!(e >= 0.f)) return 0;                            // NaN
+    return (unsigned long long)(fminf(e, 1.0f) * 1099511627776.0f);       // 2^40: the product is exact
+}
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of `p` (this block's shared memory) in block `rank` of the cluster
+template <typename V> __device__ __forceinline__ V* peer(V* p, uint32_t rank) {
+    V* r;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+    return r;
+}
+
+// exclusive prefix sum over the block's threads; *total: the sum of all
+__device__ unsigned long long block_excl_scan(unsigned long long v, unsigned long long* sh, unsigned long long* total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned long long inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long n = __shfl_up_sync(0xffffffffu, inc, o);
+        const unsigned long long n = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += n;
     }
     if (lane == 31) sh[w] = inc;
     __syncthreads();
     if (w == 0) {
-        unsigned long long x = sh[lane], xi = x;
+        const unsigned long long x = lane < SWARPS ? sh[lane] : 0;
+        unsigned long long xi = x;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long n = __shfl_up_sync(0xffffffffu, xi, o);
+        for (int o = 1; o < SWARPS; o <<= 1) {
+            const unsigned long long n = __shfl_up_sync(0xffffffffu, xi, o);
             if (lane >= o) xi += n;
         }
-        sh[lane] = xi - x;
-        if (lane == 31) sh[32] = xi;
+        if (lane < SWARPS) sh[lane] = xi - x;
+        if (lane == SWARPS - 1) sh[SWARPS] = xi;
     }
     __syncthreads();
-    unsigned long long r = sh[w] + inc - v;
-    *total = sh[32];
+    const unsigned long long r = sh[w] + inc - v;
+    *total = sh[SWARPS];
     __syncthreads();
     return r;
 }
 
-__device__ __forceinline__ unsigned long long mass_fp(float logit, float mx, float inv_t) {
-    float e = expf((logit - mx) * inv_t);
-    if (!(e >= 0.f)) return 0;                                            // NaN
-    return (unsigned long long)((double)fminf(e, 1.0f) * 1099511627776.0);   // 2^40
-}
-
-__global__ void __launch_bounds__(SB)
-sample_kernel(const float* __restrict__ logits, long long ld, int V, int* __restrict__ out,
-              float temperature, int top_k, float top_p, unsigned long long seed,
-              const int* __restrict__ keys, const int* __restrict__ steps) {
-    __shared__ ArgMax red[32];
-    __shared__ unsigned int cnt[256];
-    __shared__ unsigned long long mass[256];
-    __shared__ unsigned long long scan_sh[33];
-    __shared__ unsigned int sh_prefix, sh_krem;
-    __shared__ unsigned long long sh_acc;
-    const float* row = logits + (size_t)blockIdx.x * ld;
-    const int tid = threadIdx.x;
+// STAGED: the block's share lies in shared memory as order keys.  Otherwise (a vocabulary beyond eight blocks' shared
+// memory) every pass reads it from global memory.
+template <bool STAGED>
+__global__ void __launch_bounds__(ST, 2)
+sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, int* __restrict__ out, float temperature, int top_k,
+              float top_p, unsigned long long seed, const int* __restrict__ keys, const int* __restrict__ steps) {
+    extern __shared__ __align__(16) uint8_t sample_smem[];
+    SampleShared& sh = *reinterpret_cast<SampleShared*>(sample_smem);
+    uint32_t* staged = reinterpret_cast<uint32_t*>(sample_smem + sizeof(SampleShared));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = blockIdx.x / SC;
+    uint32_t me;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(me));
+    const int lo = min(V, (int)me * chunk), n = min(V, lo + chunk) - lo;          // this block's share of the row
+    const float* row = logits + (size_t)r * ld + lo;
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");         // (waited for before the first exchange)
     llb_grid_dependency_sync();
 
-    ArgMax top = block_argmax(row, V, red);
-    if (top_k == 1 || temperature == 0.f) {
-        if (tid == 0) out[blockIdx.x] = top.i;
+    if (STAGED) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(staged);
+        int done = 0;
+        if (((uintptr_t)row & 15) == 0) {
+            done = n & ~3;
+            for (int i = tid * 4; i < done; i += ST * 4)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 4), "l"(row + i) : "memory");
+        }
+        for (int i = done + tid; i < n; i += ST)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + i * 4), "l"(row + i) : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
+    auto key_at = [&](int i) { return STAGED ? staged[i] : order_key(row[i]); };
+
+    // ---- the maximum (the first of equals; a NaN only where there is nothing else), and every warp's largest key
+    {
+        ArgMax best = {-INFINITY, INT_MAX};
+        uint32_t top_key = 0;
+        for (int i = tid; i < n; i += ST) {
+            const float v = STAGED ? __uint_as_float(staged[i]) : row[i];
+            const uint32_t k = order_key(v);
+            if (STAGED) staged[i] = k;
+            top_key = max(top_key, k);
+            if (v > best.v || (v == v && best.i == INT_MAX)) best = {v, lo + i};     // increasing i: the first maximum stays
+        }
+        top_key = __reduce_max_sync(0xffffffffu, top_key);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const ArgMax other = {__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+            best = better(best, other);
+        }
+        if (lane == 0) sh.red[warp] = best;
+        __syncthreads();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // all blocks of the row run
+        if (lane < SC) *peer(&sh.peer_warp_max[me * SWARPS + warp], lane) = top_key;
+        if (tid < SC) {
+            ArgMax b = sh.red[0];
+            for (int w = 1; w < SWARPS; ++w) b = better(b, sh.red[w]);
+            *peer(&sh.peer_max[me], tid) = b;
+        }
+        cluster_sync();
+    }
+    ArgMax top = sh.peer_max[0];
+#pragma unroll
+    for (int c = 1; c < SC; ++c) top = better(top, sh.peer_max[c]);
+    if (top.i == INT_MAX) top.i = 0;                                              // nothing but NaN
+    if (top_k == 1 || temperature == 0.f) {                                       // (no block reads another's memory from here on)
+        if (me == 0 && tid == 0) out[r] = top.i;
         return;
     }
     const float mx = top.v, inv_t = 1.0f / temperature;
+
+    // f(key) for every key of the share with from <= key <= to
+    auto sweep = [&](uint32_t from, uint32_t to, auto f) {
+        const uint32_t span = to - from;
+        int done = 0;
+        if (STAGED) {
+            const uint4* q4 = reinterpret_cast<const uint4*>(staged);
+            done = n & ~3;
+#pragma unroll 2
+            for (int i = tid; i < done / 4; i += ST) {
+                const uint4 q = q4[i];
+                if (q.x - from <= span) f(q.x);
+                if (q.y - from <= span) f(q.y);
+                if (q.z - from <= span) f(q.z);
+                if (q.w - from <= span) f(q.w);
+            }
+        }
+        for (int i = done + tid; i < n; i += ST) {
+            const uint32_t k = key_at(i);
+            if (k - from <= span) f(k);
+        }
+    };
+    // the cluster's sum of the blocks' values v (the same in all threads of a block); below: the sum over lower blocks
+    auto cluster_sum = [&](int slot, unsigned long long v, unsigned long long* below) {
+        if (tid < SC) *peer(&sh.peer_sum[slot][me], tid) = v;
+        cluster_sync();
+        unsigned long long all = 0, b = 0;
+#pragma unroll
+        for (int c = 0; c < SC; ++c) {
+            all += sh.peer_sum[slot][c];
+            if (c < (int)me) b += sh.peer_sum[slot][c];
+        }
+        if (below) *below = b;
+        return all;
+    };
+    // Digit p of a descent (11, 11 and 10 bits) over the keys from..to whose higher digits are `prefix`; none if from > to.  By count:
+    // the digit in which the want-th largest of them lies.  By mass: the lowest digit with elements whose greater keys weigh less
+    // than `want`, `acc` of it above these keys already; `extra` elements of key extra_key count too (the owner of its bin
+    // adds them).  Leaves sh.digit, sh.above, sh.acc.
+    auto digit = [&](int p, uint32_t prefix, uint32_t from, uint32_t to, bool by_mass, unsigned long long want, unsigned long long acc,
+                     uint32_t extra_key, uint32_t extra, unsigned long long extra_mass) {
+        const int shift = p == 0 ? 21 : p == 1 ? 10 : 0, bits = p == 2 ? 10 : 11;
+        const uint32_t mask = (1u << bits) - 1;
+        for (int i = tid; i < BINS; i += ST) {
+            sh.cnt[i] = 0;
+            if (by_mass) sh.mass[0][i] = sh.mass[1][i] = sh.mass[2][i] = 0;
+        }
+        if (tid == 0) sh.lowest = SLICE;
+        __syncthreads();
+        if (from <= to) sweep(from, to, [&](uint32_t k) {
+            const uint32_t d = (k >> shift) & mask;
+            atomicAdd(&sh.cnt[d], 1u);
+            if (by_mass) {
+                const unsigned long long m = mass_fp(key_value(k), mx, inv_t);
+                if (!STAGED) {
+                    atomicAdd(&sh.whole_mass[d], m);
+                } else if (m) {
+                    atomicAdd(&sh.mass[0][d], (uint32_t)m & 0x3fffu);
+                    atomicAdd(&sh.mass[1][d], (uint32_t)(m >> 14) & 0x3fffu);
+                    atomicAdd(&sh.mass[2][d], (uint32_t)(m >> 28));
+                }
+            }
+        });
+        cluster_sync();
+        // this block's slice, the highest digit first
+        const uint32_t d = me * SLICE + SLICE - 1 - tid;
+        unsigned long long c = 0, m = 0;
+        if (tid < SLICE) {
+#pragma unroll
+            for (int q = 0; q < SC; ++q) {
+                c += *peer(&sh.cnt[d], q);
+                if (by_mass)
+                    m += STAGED ? *peer(&sh.mass[0][d], q) + ((unsigned long long)*peer(&sh.mass[1][d], q) << 14) +
+                                      ((unsigned long long)*peer(&sh.mass[2][d], q) << 28)
+                                : *peer(&sh.whole_mass[d], q);
+            }
+            if (by_mass && extra && (extra_key >> shift >> bits) == prefix && d == ((extra_key >> shift) & mask)) {
+                c += extra;
+                m += extra_mass;
+            }
+        }
+        unsigned long long c_all, m_all = 0, m_above = 0;
+        unsigned long long c_above = block_excl_scan(c, sh.scan, &c_all);
+        if (by_mass) m_above = block_excl_scan(m, sh.scan, &m_all);
+        if (tid < SC) {
+            *peer(&sh.peer_cnt[me], tid) = c_all;
+            *peer(&sh.peer_mass[me], tid) = m_all;
+        }
+        cluster_sync();
+        unsigned long long c_base = 0, m_base = acc;                              // above this slice
+        for (int q = SC - 1; q > (int)me; --q) { c_base += sh.peer_cnt[q]; m_base += sh.peer_mass[q]; }
+        bool mine;
+        if (by_mass) {
+            mine = c > 0 && m_base + m_above < want;
+            // a lower slice with elements that still qualifies comes before this one
+            unsigned long long below = m_base + sh.peer_mass[me];
+            for (int q = (int)me - 1; q >= 0; --q) {
+                if (sh.peer_cnt[q] && below < want) mine = false;
+                below += sh.peer_mass[q];
+            }
+            if (mine) atomicMin(&sh.lowest, (uint32_t)(SLICE - 1 - tid));
+            __syncthreads();
+            mine = mine && sh.lowest == (uint32_t)(SLICE - 1 - tid);
+        } else {
+            mine = tid < SLICE && c_base + c_above < want && want <= c_base + c_above + c;
+        }
+        if (mine)
+            for (int q = 0; q < SC; ++q) {
+                *peer(&sh.digit, q) = d;
+                *peer(&sh.above, q) = (uint32_t)(c_base + c_above);
+                *peer(&sh.acc, q) = m_base + m_above;
+            }
+        cluster_sync();
+    };
+    // digit p's keys for the digits chosen so far: the lowest and the highest, and the prefix with one more digit
+    auto lowest_of = [](int p, uint32_t prefix) { return p == 0 ? 0u : p == 1 ? prefix << 21 : prefix << 10; };
+    auto highest_of = [](int p, uint32_t prefix) { return p == 0 ? UINT_MAX : p == 1 ? (prefix << 21) | 0x1fffffu : (prefix << 10) | 0x3ffu; };
+    auto append = [](int p, uint32_t prefix, uint32_t d) { return p == 2 ? (prefix << 10) | d : (prefix << 11) | d; };
 
     // ---- top-k: the k-th largest key and how many of its equals are admitted
     uint32_t kth_key = 0;
     unsigned int ties_k = UINT_MAX;
     if (top_k > 0 && top_k < V) {
-        if (tid == 0) { sh_prefix = 0; sh_krem = (unsigned)top_k; }
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            if (tid < 256) cnt[tid] = 0;
-            __syncthreads();
-            uint32_t prefix = sh_prefix;
-            for (int i = tid; i < V; i += SB) {
-                uint32_t k = order_key(row[i]);
-                if (shift == 24 || (k >> (shift + 8)) == prefix) atomicAdd(&cnt[(k >> shift) & 255u], 1u);
-            }
-            __syncthreads();
-            if (tid == 0) {
-                unsigned int rem = sh_krem, above = 0;
-                int d = 255;
-                for (; d > 0; --d) {
-                    if (above + cnt[d] >= rem) break;
-                    above += cnt[d];
+        // At least top_k elements reach the top_k-th largest of the warps' maxima: what is below it need not be counted.
+        uint32_t floor_key = 0;
+        if (top_k <= SC * SWARPS) {
+            if (tid < SC * SWARPS) {
+                const uint32_t v = sh.peer_warp_max[tid];
+                int greater = 0, reach = 0;
+                for (int w = 0; w < SC * SWARPS; ++w) {
+                    greater += sh.peer_warp_max[w] > v;
+                    reach += sh.peer_warp_max[w] >= v;
                 }
-                sh_krem = rem - above;
-                sh_prefix = (prefix << 8) | (unsigned)d;
+                if (greater < top_k && top_k <= reach) sh.floor_key = v;          // (equal values write the same)
             }
             __syncthreads();
+            floor_key = sh.floor_key;
         }
-        kth_key = sh_prefix;
-        ties_k = sh_krem;
+        uint32_t prefix = 0, rem = (uint32_t)top_k;
+#pragma unroll 1
+        for (int p = 0; p < 3; ++p) {
+            digit(p, prefix, max(lowest_of(p, prefix), floor_key), highest_of(p, prefix), false, rem, 0, 0, 0, 0);
+            rem -= sh.above;
+            prefix = append(p, prefix, sh.digit);
+        }
+        kth_key = prefix;
+        ties_k = rem;
     }
 
-    // ---- kept mass after top-k
+    // ---- top-p: of these, the lowest key and how many of its equals are needed to reach the mass
     uint32_t cut_key = kth_key;
     unsigned int ties = ties_k;
-    unsigned long long kth_mass = mass_fp(key_value(kth_key), mx, inv_t);
     if (top_p < 1.0f) {
-        unsigned long long part = 0;
-        for (int i = tid; i < V; i += SB) {
-            float v = row[i];
-            if (order_key(v) > kth_key) part += mass_fp(v, mx, inv_t);
-        }
-        unsigned long long zk;
-        block_excl_scan(part, scan_sh, &zk);
+        const unsigned long long kth_mass = mass_fp(key_value(kth_key), mx, inv_t);
+        unsigned long long part = 0, own, equal = 0;
+        if (kth_key < UINT_MAX) sweep(kth_key + 1, UINT_MAX, [&](uint32_t k) { part += mass_fp(key_value(k), mx, inv_t); });
+        block_excl_scan(part, sh.scan, &own);
+        unsigned long long zk = cluster_sum(0, own, nullptr);
         unsigned int n_eq_kept = ties_k;
         if (ties_k == UINT_MAX) {             // no top-k: every element equal to the minimum key counts
-            unsigned long long c = 0;
-            for (int i = tid; i < V; i += SB) c += order_key(row[i]) == kth_key;
-            unsigned long long tot;
-            block_excl_scan(c, scan_sh, &tot);
-            n_eq_kept = (unsigned)tot;
+            sweep(kth_key, kth_key, [&](uint32_t) { ++equal; });
+            block_excl_scan(equal, sh.scan, &own);
+            n_eq_kept = (unsigned)cluster_sum(1, own, nullptr);
         }
         zk += (unsigned long long)n_eq_kept * kth_mass;
-        unsigned long long target = (unsigned long long)ceil((double)top_p * (double)zk);
+        unsigned long long target = (unsigned long long)ceil((double)top_p * (double)zk), acc = 0;
         if (target < 1) target = 1;
-
-        // radix descent by mass: the lowest key whose mass of greater kept keys is below target
-        if (tid == 0) { sh_prefix = 0; sh_acc = 0; }
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            if (tid < 256) { cnt[tid] = 0; mass[tid] = 0; }
-            __syncthreads();
-            uint32_t prefix = sh_prefix;
-            for (int i = tid; i < V; i += SB) {
-                float v = row[i];
-                uint32_t k = order_key(v);
-                if (k > kth_key && (shift == 24 || (k >> (shift + 8)) == prefix)) {
-                    atomicAdd(&cnt[(k >> shift) & 255u], 1u);
-                    atomicAdd(&mass[(k >> shift) & 255u], mass_fp(v, mx, inv_t));
-                }
-            }
-            if (tid == 0 && n_eq_kept > 0 && (shift == 24 || (kth_key >> (shift + 8)) == prefix)) {
-                atomicAdd(&cnt[(kth_key >> shift) & 255u], n_eq_kept);
-                atomicAdd(&mass[(kth_key >> shift) & 255u], (unsigned long long)n_eq_kept * kth_mass);
-            }
-            __syncthreads();
-            if (tid == 0) {
-                unsigned long long running = sh_acc, chosen_acc = sh_acc;
-                int chosen = -1;
-                for (int d = 255; d >= 0; --d) {
-                    if (running >= target) break;
-                    if (cnt[d] > 0) { chosen = d; chosen_acc = running; }
-                    running += mass[d];
-                }
-                if (chosen < 0) chosen = 255;
-                sh_prefix = (prefix << 8) | (unsigned)chosen;
-                sh_acc = chosen_acc;
-            }
-            __syncthreads();
+        uint32_t prefix = 0;
+#pragma unroll 1
+        for (int p = 0; p < 3; ++p) {
+            // the kept keys above kth_key; its own equals go in as extra elements
+            const uint32_t to = highest_of(p, prefix);
+            const bool any = kth_key < to;
+            digit(p, prefix, any ? max(lowest_of(p, prefix), kth_key + 1) : 1, any ? to : 0, true, target, acc, kth_key, n_eq_kept,
+                  (unsigned long long)n_eq_kept * kth_mass);
+            acc = sh.acc;
+            prefix = append(p, prefix, sh.digit);
         }
-        cut_key = sh_prefix;
-        unsigned long long acc = sh_acc;
-        unsigned long long cm = mass_fp(key_value(cut_key), mx, inv_t);
-        unsigned long long need = target > acc ? target - acc : 1;
+        cut_key = prefix;
+        const unsigned long long cm = mass_fp(key_value(cut_key), mx, inv_t);
+        const unsigned long long need = target > acc ? target - acc : 1;
         unsigned long long n_ties_p = cm > 0 ? (need + cm - 1) / cm : (unsigned long long)UINT_MAX;
         if (n_ties_p > UINT_MAX) n_ties_p = UINT_MAX;
         ties = (unsigned)n_ties_p;
@@ -316,44 +494,67 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int* __rest
     }
     const unsigned long long cut_mass = mass_fp(key_value(cut_key), mx, inv_t);
 
-    // ---- draw over the kept set in index order; thread t owns one contiguous segment
-    const int seg = (V + SB - 1) / SB;
-    const int lo = min(V, tid * seg), hi = min(V, lo + seg);
-    unsigned long long eq = 0;
-    for (int i = lo; i < hi; ++i) eq += order_key(row[i]) == cut_key;
-    unsigned long long eq_total;
-    unsigned long long eq_base = block_excl_scan(eq, scan_sh, &eq_total);
+    // ---- draw over the kept set in index order; thread t owns one contiguous segment of the share (of odd length: no bank conflicts)
+    const int seg = ((n + ST - 1) / ST) | 1;
+    const int from = min(n, tid * seg), to = min(n, from + seg);
+    unsigned long long eq = 0, eq_own, eq_base;
+    for (int i = from; i < to; ++i) eq += key_at(i) == cut_key;
+    const unsigned long long eq_before = block_excl_scan(eq, sh.scan, &eq_own);
+    cluster_sum(2, eq_own, &eq_base);
+    eq_base += eq_before;
     unsigned long long seg_mass = 0, rank = eq_base;
-    for (int i = lo; i < hi; ++i) {
-        float v = row[i];
-        uint32_t k = order_key(v);
-        if (k > cut_key) seg_mass += mass_fp(v, mx, inv_t);
+    for (int i = from; i < to; ++i) {
+        const uint32_t k = key_at(i);
+        if (k > cut_key) seg_mass += mass_fp(key_value(k), mx, inv_t);
         else if (k == cut_key) { if (rank < ties) seg_mass += cut_mass; ++rank; }
     }
-    unsigned long long total;
-    unsigned long long before = block_excl_scan(seg_mass, scan_sh, &total);
+    unsigned long long own_mass, before;
+    const unsigned long long before_own = block_excl_scan(seg_mass, sh.scan, &own_mass);
+    const unsigned long long total = cluster_sum(3, own_mass, &before);           // (the last exchange)
+    before += before_own;
     if (total == 0) {                      // every kept mass underflowed: fall back to the maximum
-        if (tid == 0) out[blockIdx.x] = top.i;
+        if (me == 0 && tid == 0) out[r] = top.i;
         return;
     }
-    double u = llb_uniform(seed, (unsigned long long)(keys ? keys[blockIdx.x] : blockIdx.x),
-                           (unsigned long long)(steps ? steps[blockIdx.x] : 0));
+    const double u = llb_uniform(seed, (unsigned long long)(keys ? keys[r] : r), (unsigned long long)(steps ? steps[r] : 0));
     unsigned long long target = (unsigned long long)(u * (double)total);
     if (target >= total) target = total - 1;
     if (target >= before && target < before + seg_mass) {
         unsigned long long run = before, rk = eq_base;
-        int pick = lo;
-        for (int i = lo; i < hi; ++i) {
-            float v = row[i];
-            uint32_t k = order_key(v);
-            unsigned long long mfp = 0;
-            if (k > cut_key) mfp = mass_fp(v, mx, inv_t);
-            else if (k == cut_key) { if (rk < ties) mfp = cut_mass; ++rk; }
-            if (mfp > 0 && target < run + mfp) { pick = i; break; }
-            run += mfp;
+        int pick = from;
+        for (int i = from; i < to; ++i) {
+            const uint32_t k = key_at(i);
+            unsigned long long m = 0;
+            if (k > cut_key) m = mass_fp(key_value(k), mx, inv_t);
+            else if (k == cut_key) { if (rk < ties) m = cut_mass; ++rk; }
+            if (m > 0 && target < run + m) { pick = i; break; }
+            run += m;
         }
-        out[blockIdx.x] = pick;
+        out[r] = lo + pick;
     }
+}
+
+template <bool STAGED, typename... A>
+static int launch_sample(int R, size_t smem, cudaStream_t stream, A... args) {
+    auto kernel = sample_kernel<STAGED>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGED ? SMEM_MAX : (int)smem);
+    if (e != cudaSuccess) return -2000 - (int)e;
+    llb_prefer_max_shared((const void*)kernel);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)R * SC);
+    cfg.blockDim = dim3(ST);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SC;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = llb_pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    return llb_status();
 }
 
 // keys[r], steps[r]: the request number and the count of tokens already drawn for row r; they
@@ -362,9 +563,12 @@ LLB_API int llb_sample(const float* logits, long long ld, int R, int V, int* out
                        int top_k, float top_p, unsigned long long seed, const int* keys,
                        const int* steps, cudaStream_t stream) {
     if (R == 0) return 0;
-    if (V <= 0 || temperature < 0.f || !(top_p > 0.f)) return (int)cudaErrorInvalidValue;
-    llb_launch(sample_kernel, dim3(R), dim3(SB), 0, stream, logits, ld, V, out, temperature, top_k, top_p, seed, keys, steps);
-    return llb_status();
+    if (V <= 0 || temperature < 0.f || !(top_p > 0.f) || R > INT_MAX / SC) return (int)cudaErrorInvalidValue;
+    const int chunk = ((V + SC - 1) / SC + 3) & ~3;                               // whole 16-byte pieces
+    const size_t smem = sizeof(SampleShared) + (size_t)chunk * 4;
+    if (smem <= SMEM_MAX)
+        return launch_sample<true>(R, smem, stream, logits, ld, V, chunk, out, temperature, top_k, top_p, seed, keys, steps);
+    return launch_sample<false>(R, sizeof(SampleShared), stream, logits, ld, V, chunk, out, temperature, top_k, top_p, seed, keys, steps);
 }
 
 LLB_API double llb_uniform_host(unsigned long long seed, unsigned long long key, unsigned long long step) {
