@@ -59,6 +59,7 @@ constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 constexpr uint64_t HINT_EVICT_FIRST = 0x12F0000000000000ull;
 constexpr uint64_t HINT_EVICT_LAST = 0x14F0000000000000ull;
+constexpr uint64_t HINT_EVICT_NORMAL = 0x1000000000000000ull;
 
 enum { ERR_TC2_WAIT_FULL = 111, ERR_TC2_WAIT_EMPTY = 112, ERR_TC2_WAIT_ACC_FULL = 113, ERR_TC2_WAIT_ACC_EMPTY = 114 };
 
@@ -163,9 +164,21 @@ struct Gemm2Args {
     int rows_out;          // N, or the number of gate rows with DUAL
     int dual_offset;
     int tok_tiles, n_tiles, n_pairs;
+    int group, row_tiles;  // the order of the tiles: see Gemm2Args::place
+    uint64_t hint_w, hint_x;
     int* err;
     int ksplit, chunk_kb;  // INTO: K ranges per tile and k-blocks per range (1 and all of them otherwise)
     GluForm glu = {};      // DUAL: how gate and up combine
+
+    // Tile t's block of weight rows and its block of tokens.  Tiles are walked in bands of `group` weight blocks: inside a band the
+    // weight block changes first, then the token block, so that the tiles which the pairs work on at one time form a
+    // rectangle and not a strip.
+    __device__ __forceinline__ void place(int t, int& row_tile, int& tok_tile) const {
+        const int band = t / (group * tok_tiles), in_band = t - band * group * tok_tiles;
+        const int rows = min(group, row_tiles - band * group);
+        tok_tile = in_band / rows;
+        row_tile = band * group + in_band - tok_tile * rows;
+    }
 };
 
 // The loads issued so far have arrived.  The registers pass through the statement so that no use of them is
@@ -259,12 +272,14 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int prefetched = min(STAGES, unit_kb1(pair) - first_kb0);
     if (warp == 0 && lane == 0) {
         const uint32_t full0 = mapa(bar_full, 0);
-        const int m0 = (((pair % g.n_tiles) / g.tok_tiles) * 2 + (int)rank) * MROWS;
+        int row_tile, tok_tile;
+        g.place(pair % g.n_tiles, row_tile, tok_tile);
+        const int m0 = (row_tile * 2 + (int)rank) * MROWS;
         for (int i = 0; i < prefetched; ++i) {
             const uint32_t dst = base + i * S::STAGE_BYTES, bar = full0 + 8 * i;
             if (leader) mbar_expect_tx(bar_full + 8 * i, 2u * S::STAGE_BYTES);
-            tma_load_2d_pair(dst, &map_w, bar, (first_kb0 + i) * BK, m0, HINT_EVICT_FIRST);      // DUAL 1: the map's box is 64 rows
-            if (DUAL) tma_load_2d_pair(dst + S::A_BYTES / (3 - DUAL), &map_w, bar, (first_kb0 + i) * BK, m0 + g.dual_offset, HINT_EVICT_FIRST);
+            tma_load_2d_pair(dst, &map_w, bar, (first_kb0 + i) * BK, m0, g.hint_w);      // DUAL 1: the map's box is 64 rows
+            if (DUAL) tma_load_2d_pair(dst + S::A_BYTES / (3 - DUAL), &map_w, bar, (first_kb0 + i) * BK, m0 + g.dual_offset, g.hint_w);
         }
     }
     llb_grid_dependency_sync();      // from here on memory written by earlier kernels is touched
@@ -274,17 +289,21 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // warp waits for a free stage as a whole; one elected lane issues the copies.
         const uint32_t full0 = mapa(bar_full, 0);
         if (elect_one()) {   // the activations of the k-blocks whose weight is on its way already
-            const int n0 = ((pair % g.n_tiles) % g.tok_tiles) * BN + (int)rank * (BN / 2);
+            int row_tile, tok_tile;
+            g.place(pair % g.n_tiles, row_tile, tok_tile);
+            const int n0 = tok_tile * BN + (int)rank * (BN / 2);
             for (int i = 0; i < prefetched; ++i)
-                tma_load_2d_pair(base + i * S::STAGE_BYTES + ACCS * S::A_BYTES, &map_x, full0 + 8 * i, (first_kb0 + i) * BK, n0, HINT_EVICT_LAST);
+                tma_load_2d_pair(base + i * S::STAGE_BYTES + ACCS * S::A_BYTES, &map_x, full0 + 8 * i, (first_kb0 + i) * BK, n0, g.hint_x);
         }
         __syncwarp();
         int it = prefetched;
         bool ok = true;
         for (int u = pair; u < n_units && ok; u += g.n_pairs) {
-            const int t = u % g.n_tiles, kb1 = unit_kb1(u);
-            const int m0 = ((t / g.tok_tiles) * 2 + (int)rank) * MROWS;
-            const int n0 = (t % g.tok_tiles) * BN + (int)rank * (BN / 2);
+            const int kb1 = unit_kb1(u);
+            int row_tile, tok_tile;
+            g.place(u % g.n_tiles, row_tile, tok_tile);
+            const int m0 = (row_tile * 2 + (int)rank) * MROWS;
+            const int n0 = tok_tile * BN + (int)rank * (BN / 2);
             for (int kb = unit_kb0(u) + (u == pair ? prefetched : 0); kb < kb1; ++kb, ++it) {
                 const int s = it % STAGES;
                 if (it >= STAGES && !warp_wait(bar_empty + 8 * s, (uint32_t)(it / STAGES - 1) & 1u, &s_abort)) {
@@ -295,9 +314,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (elect_one()) {
                     const uint32_t dst = base + s * S::STAGE_BYTES, bar = full0 + 8 * s;
                     if (leader) mbar_expect_tx(bar_full + 8 * s, 2u * S::STAGE_BYTES);
-                    tma_load_2d_pair(dst, &map_w, bar, kb * BK, m0, HINT_EVICT_FIRST);
-                    if (DUAL) tma_load_2d_pair(dst + S::A_BYTES / (3 - DUAL), &map_w, bar, kb * BK, m0 + g.dual_offset, HINT_EVICT_FIRST);
-                    tma_load_2d_pair(dst + ACCS * S::A_BYTES, &map_x, bar, kb * BK, n0, HINT_EVICT_LAST);
+                    tma_load_2d_pair(dst, &map_w, bar, kb * BK, m0, g.hint_w);
+                    if (DUAL) tma_load_2d_pair(dst + S::A_BYTES / (3 - DUAL), &map_w, bar, kb * BK, m0 + g.dual_offset, g.hint_w);
+                    tma_load_2d_pair(dst + ACCS * S::A_BYTES, &map_x, bar, kb * BK, n0, g.hint_x);
                 }
                 __syncwarp();
             }
@@ -373,9 +392,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const bool stamper = tid == (DUAL == 1 ? 128 : 64);       // (a storing warp's first thread)
         int ti = 0, chunk_i = 0;
         for (int u = pair; u < n_units; u += g.n_pairs, ++ti) {
-            const int buf = ti % NBUF, t = u % g.n_tiles;
-            const int m0 = ((t / g.tok_tiles) * 2 + (int)rank) * MROWS;
-            const int n0 = (t % g.tok_tiles) * BN;
+            const int buf = ti % NBUF;
+            int row_tile, tok_tile;
+            g.place(u % g.n_tiles, row_tile, tok_tile);
+            const int m0 = (row_tile * 2 + (int)rank) * MROWS;
+            const int n0 = tok_tile * BN;
             const int m = m0 + row;
             float bias_v = 0.f;
             if (!DUAL && g.bias && m < g.rows_out && u < g.n_tiles)    // the bias goes in with the first K range only
@@ -532,6 +553,24 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, 
 
 LLB_DEFINE_SET_STAMPS
 
+// The order of the tiles.  Up to sixteen blocks of tokens a weight block meets all of them at one time (bands of one weight block: the
+// pairs' tiles are about square by themselves), is read once and may leave the L2 first, while the tokens stay.  With more, the pairs
+// at work would all sit on one or two weight blocks and stream as many token blocks as there are pairs from memory, once
+// per weight block; bands of about eight weight blocks keep the rectangle near square, and both operands are kept as
+// the L2 sees fit.  Measured (gate/up, down, q/k/v of the 7B shape back to back, us): 34,816 tokens 13,330 -> 11,600, 8,192 tokens
+// 2,520 -> 2,350, 4,096 tokens 1,181 -> 1,195; alone at 34,816 tokens 7,480 -> 5,970, 4,140 -> 2,960, 946 -> 709.
+static void set_order(Gemm2Args& g, int row_tiles) {
+    g.row_tiles = row_tiles;
+    g.group = 1;
+    g.hint_w = HINT_EVICT_FIRST;
+    g.hint_x = HINT_EVICT_LAST;
+    if (g.tok_tiles > 16) {
+        const int bands = (row_tiles + 4) / 8 < 1 ? 1 : (row_tiles + 4) / 8;
+        g.group = (row_tiles + bands - 1) / bands;
+        g.hint_w = g.hint_x = HINT_EVICT_NORMAL;
+    }
+}
+
 // X [T, K] bf16 with row stride ldx; W [N, K] bf16 dense ([2 * dual_offset, K] when dual_offset > 0); Y [T, ldy]
 // bf16; bias [N] or null.  max_pairs: how many CTA pairs may run at once (SMs / 2).  Returns
 // cudaErrorInvalidValue for what this kernel does not take (the caller then uses the one-CTA kernel).
@@ -548,15 +587,16 @@ LLB_API int llb_gemm_tc2(const void* X, const void* W, const void* bias, int bia
     Gemm2Args g;
     g.bias = bias; g.bias_dtype = bias_dtype; g.Y = (bf16*)Y;
     g.T = T; g.K = K; g.ldy = ldy; g.rows_out = rows_out; g.dual_offset = dual_offset;
-    g.tok_tiles = (T + bn - 1) / bn;
     // gate/up: with a short K range the one-accumulator variant, whose epilogue runs beside the next tile's products
     // (64 gate and 64 up rows per CTA); with a long one the two-accumulator variant, which takes a third less from the
     // L2 per FLOP and loses little to its exposed epilogue (a prefill step of 2,048 tokens with the first variant: 4 %
     // shorter at K 1536, I 8960; 4 % longer at K 3584, I 18944; the same at K 5120, I 27648).
     const bool side_by_side = dual && K <= 2048;
     const int tile_rows = side_by_side ? BM : 2 * BM;  // output rows of a pair's tile
+    g.tok_tiles = (T + bn - 1) / bn;
     const long long tiles = (long long)((rows_out + tile_rows - 1) / tile_rows) * g.tok_tiles;
     if (tiles > (1 << 30)) return (int)cudaErrorInvalidValue;
+    set_order(g, (rows_out + tile_rows - 1) / tile_rows);
     g.n_tiles = (int)tiles;
     g.n_pairs = (int)(tiles < max_pairs ? tiles : max_pairs);
     g.err = err;
@@ -609,6 +649,7 @@ LLB_API int llb_gemm_tc2_into(const void* X, const void* W, const void* bias, in
     g.tok_tiles = (T + bn - 1) / bn;
     const long long tiles = (long long)((N + 2 * BM - 1) / (2 * BM)) * g.tok_tiles;
     if (tiles * ksplit > (1 << 30)) return (int)cudaErrorInvalidValue;
+    set_order(g, (N + 2 * BM - 1) / (2 * BM));
     g.n_tiles = (int)tiles;
     g.chunk_kb = (kblocks + ksplit - 1) / ksplit;
     g.ksplit = (kblocks + g.chunk_kb - 1) / g.chunk_kb;                  // no range is empty
