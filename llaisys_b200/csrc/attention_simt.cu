@@ -93,6 +93,8 @@ struct AttnParams {
     float softcap;        // > 0: scaled scores pass through softcap * tanh(. / softcap)
 };
 
+template <int V> struct IntC { static constexpr int value = V; };
+
 template <typename T, bool DECODE>
 __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
     extern __shared__ float smem[];
@@ -179,8 +181,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
         const bool pooled = it < n_pool;
         const int tile = pooled ? it : (it - n_pool < n_kept ? it - n_pool : tile_lo + it - n_pool - n_kept);
         __syncthreads();                     // previous tile fully consumed (and Qs written)
-        // A tile is one cache page (tiles start at multiples of LLB_PAGE): its page is looked up once; rows move in
-        // 16-byte pieces where the widths and the addresses allow it.
+        // A tile is one cache page (tiles start at multiples of LLB_PAGE): its page is looked up once.
         const int p0 = tile * LLB_PAGE;
         // (the page table is read only for a tile that holds cached positions: a step without history may come with
         // an empty table)
@@ -200,66 +201,51 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
         const bool cached = DECODE || p.all_from_cache || p0 < len_before;
         const T* kpage = (cached && !pooled) ? kpool + paged_row(table, p.ring, p0, vh, cache_heads, krow, p.pinned) + kmap * DH : nullptr;
         constexpr int VEC = 16 / (int)sizeof(T);
-        const bool kvec = DH % VEC == 0 && (((uintptr_t)kpool | (uintptr_t)knew) & 15) == 0 && kv_stride % VEC == 0;
-        if (pooled) {
-        } else if (kvec) {
-            // eight pieces a thread are requested before the first is used: the walk waits for memory once per batch
-            constexpr int PIECES = LLB_PAGE * (DH / VEC), BATCH = 8;
-            for (int i0 = tid; i0 < PIECES; i0 += BATCH * WARPS * 32) {
-                uint4 raw[BATCH];
+        // One tile of rows of WIDTH elements into shared memory (row stride `pitch` floats): in 16-byte pieces where the width and
+        // the addresses allow it, as many of a thread's pieces as fit BATCH requested before the first is used, so that the
+        // walk waits for memory once per batch and not once per element.
+        auto fetch_tile = [&](auto width, float* dst, int pitch, const T* pool, const T* page, int page_row, const T* fresh, int fresh_col) {
+            constexpr int WIDTH = decltype(width)::value, PER = WIDTH / VEC > 0 ? WIDTH / VEC : 1;      // pieces of a row
+            constexpr int PIECES = LLB_PAGE * PER, SHARE = (PIECES + WARPS * 32 - 1) / (WARPS * 32);
+            constexpr int BATCH = SHARE < 16 ? SHARE : 16;
+            auto source = [&](int j, int d) -> const T* {                    // null: outside what the block sees
+                const int kp = p0 + j;
+                if (!((kp >= key_lo || kp < keep) && kp <= last_pos)) return nullptr;
+                return (!DECODE && !p.all_from_cache && kp >= len_before)
+                           ? fresh + (size_t)(tok0 + kp - len_before) * kv_stride + fresh_col + d
+                           : page + (size_t)j * page_row + d;
+            };
+            if (WIDTH % VEC == 0 && (((uintptr_t)pool | (uintptr_t)fresh) & 15) == 0 && kv_stride % VEC == 0) {
+                for (int i0 = tid; i0 < PIECES; i0 += BATCH * WARPS * 32) {
+                    uint4 raw[BATCH];
 #pragma unroll
-                for (int u = 0; u < BATCH; ++u) {
-                    const int i = i0 + u * WARPS * 32;
-                    raw[u] = make_uint4(0u, 0u, 0u, 0u);                 // zero bits are zero in both types
-                    if (i < PIECES) {
-                        const int j = i / (DH / VEC), d = (i - j * (DH / VEC)) * VEC, kp = p0 + j;
-                        if ((kp >= key_lo || kp < keep) && kp <= last_pos) {
-                            const T* src = (!DECODE && !p.all_from_cache && kp >= len_before)
-                                               ? knew + (size_t)(tok0 + kp - len_before) * kv_stride + kvh * DH + d
-                                               : kpage + (size_t)j * krow + d;
-                            raw[u] = *reinterpret_cast<const uint4*>(src);
-                        }
+                    for (int u = 0; u < BATCH; ++u) {
+                        const int i = i0 + u * WARPS * 32, j = i / PER, d = (i - j * PER) * VEC;
+                        const T* src = i < PIECES ? source(j, d) : nullptr;
+                        raw[u] = src ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);     // zero bits are zero in both types
                     }
-                }
 #pragma unroll
-                for (int u = 0; u < BATCH; ++u) {
-                    const int i = i0 + u * WARPS * 32;
-                    if (i < PIECES) {
-                        const int j = i / (DH / VEC), d = (i - j * (DH / VEC)) * VEC;
+                    for (int u = 0; u < BATCH; ++u) {
+                        const int i = i0 + u * WARPS * 32, j = i / PER, d = (i - j * PER) * VEC;
                         const T* rv = reinterpret_cast<const T*>(&raw[u]);
+                        if (i < PIECES)
 #pragma unroll
-                        for (int e = 0; e < VEC; ++e) Ks[j * (DH + 1) + d + e] = to_f32(rv[e]);
+                            for (int e = 0; e < VEC; ++e) dst[j * pitch + d + e] = to_f32(rv[e]);
                     }
                 }
+                return;
             }
-        } else {
-            for (int i = tid; i < LLB_PAGE * DH; i += WARPS * 32) {
-                int j = i / DH, d = i - j * DH;
-                int kp = p0 + j;
-                float kv = 0.f;
-                if ((kp >= key_lo || kp < keep) && kp <= last_pos) {
-                    if (!DECODE && !p.all_from_cache && kp >= len_before)
-                        kv = to_f32(knew[(size_t)(tok0 + kp - len_before) * kv_stride + kvh * DH + d]);
-                    else
-                        kv = to_f32(kpage[(size_t)j * krow + d]);
-                }
-                Ks[j * (DH + 1) + d] = kv;
+            for (int i = tid; i < LLB_PAGE * WIDTH; i += WARPS * 32) {
+                const int j = i / WIDTH, d = i - j * WIDTH;
+                const T* src = source(j, d);
+                dst[j * pitch + d] = src ? to_f32(*src) : 0.f;
             }
-        }
-        if (!p.v_in_k && !pooled) {
-            const T* vpage = cached ? vpool + paged_row(table, p.ring, p0, vh, cache_heads, DV, p.pinned) : nullptr;
-            for (int i = tid; i < LLB_PAGE * DV; i += WARPS * 32) {
-                int j = i / DV, d = i - j * DV;
-                int kp = p0 + j;
-                float vv = 0.f;
-                if ((kp >= key_lo || kp < keep) && kp <= last_pos) {
-                    if (!DECODE && !p.all_from_cache && kp >= len_before)
-                        vv = to_f32(vnew[(size_t)(tok0 + kp - len_before) * kv_stride + vh * DV + d]);
-                    else
-                        vv = to_f32(vpage[(size_t)j * DV + d]);
-                }
-                Vs[j * DV + d] = vv;
-            }
+        };
+        if (!pooled) {
+            fetch_tile(IntC<DH>(), Ks, DH + 1, kpool, kpage, krow, knew, kvh * DH);
+            if (!p.v_in_k)
+                fetch_tile(IntC<DV>(), Vs, DV, vpool, cached ? vpool + paged_row(table, p.ring, p0, vh, cache_heads, DV, p.pinned) : nullptr, DV,
+                           vnew, vh * DV);
         }
         __syncthreads();
 #pragma unroll
