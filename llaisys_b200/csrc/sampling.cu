@@ -165,18 +165,31 @@ LLB_API int llb_argmax_split(const float* logits, long long ld, int R, int V, in
 //
 // The rule needs a dozen passes over a row (the maximum, three digits of the k-th largest key, the kept mass, three digits of the
 // nucleus' cut, the draw).  With one block per row they all came from the L2 at one SM's rate: 571 us for 64 rows of 151,936, whose one
-// read from memory takes 6 (now 110).  Here the row is read once, the passes run over shared memory, and the blocks exchange what they
+// read from memory takes 6 (now 29, with top-k 50).  Here the row is read once, the passes run over shared memory, and the blocks exchange what they
 // must (histograms of a digit, sums) through each other's shared memory between cluster barriers.  Every sum is one of
 // integers, so how a row is divided does not change the result.
 constexpr int ST = 512, SWARPS = ST / 32, SC = 8;         // threads of a block, blocks of a row
 constexpr int BINS = 2048, SLICE = BINS / SC;             // values of a digit; a block adds up its slice of them over the cluster
+constexpr int CAP = 128;                                  // candidates of a block on the short way
 constexpr int SMEM_MAX = 232448;
 
-struct SampleShared {
+struct alignas(16) SampleShared {              // (the share behind it is read and filled in 16-byte pieces)
     // a digit's histogram over this block's elements: counts and masses.  The masses (at most 2^40 each) are added in parts of 14,
     // 14 and 13 bits while 2^18 elements a block are out of reach, because 64-bit atomics on shared memory are loops
-    uint32_t cnt[BINS];
-    union { uint32_t mass[3][BINS]; unsigned long long whole_mass[BINS]; };
+    alignas(16) uint32_t cnt[BINS];
+    // (the short way has its lists in the same place: the block's own candidates, the cluster's in block 0, and these in order)
+    union alignas(16) {
+        uint32_t mass[3][BINS];
+        unsigned long long whole_mass[BINS];
+        struct {
+            uint2 own[CAP], all[SC][CAP];
+            unsigned long long by_key[ST], by_index[ST];
+            int index[ST];
+            uint32_t kept[ST];
+        } list;
+    };
+    alignas(16) uint32_t slice_cnt[SLICE];                            // the cluster's sums of this block's slice
+    unsigned long long slice_mass[SLICE];
     unsigned long long scan[SWARPS + 1];
     // written by the cluster's blocks, read behind a cluster barrier
     ArgMax peer_max[SC];
@@ -187,8 +200,11 @@ struct SampleShared {
     unsigned long long acc;                               // ... and their mass
     // the block's own
     ArgMax red[SWARPS];
-    uint32_t floor_key, lowest;
+    uint32_t floor_key, lowest, n_own;
+    uint32_t peer_found[SC];                              // (written by the cluster's blocks) candidates of every block
 };
+
+static_assert(sizeof(SampleShared) % 16 == 0, "the share starts on a 16-byte boundary");
 
 __device__ __forceinline__ unsigned long long mass_fp(float logit, float mx, float inv_t) {
     float e = expf((logit - mx) * inv_t);
@@ -306,7 +322,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
     }
     const float mx = top.v, inv_t = 1.0f / temperature;
 
-    // f(key) for every key of the share with from <= key <= to
+    // f(key, place in the share) for every key of the share with from <= key <= to
     auto sweep = [&](uint32_t from, uint32_t to, auto f) {
         const uint32_t span = to - from;
         int done = 0;
@@ -316,15 +332,15 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
 #pragma unroll 2
             for (int i = tid; i < done / 4; i += ST) {
                 const uint4 q = q4[i];
-                if (q.x - from <= span) f(q.x);
-                if (q.y - from <= span) f(q.y);
-                if (q.z - from <= span) f(q.z);
-                if (q.w - from <= span) f(q.w);
+                if (q.x - from <= span) f(q.x, 4 * i);
+                if (q.y - from <= span) f(q.y, 4 * i + 1);
+                if (q.z - from <= span) f(q.z, 4 * i + 2);
+                if (q.w - from <= span) f(q.w, 4 * i + 3);
             }
         }
         for (int i = done + tid; i < n; i += ST) {
             const uint32_t k = key_at(i);
-            if (k - from <= span) f(k);
+            if (k - from <= span) f(k, i);
         }
     };
     // the cluster's sum of the blocks' values v (the same in all threads of a block); below: the sum over lower blocks
@@ -354,7 +370,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
         }
         if (tid == 0) sh.lowest = SLICE;
         __syncthreads();
-        if (from <= to) sweep(from, to, [&](uint32_t k) {
+        if (from <= to) sweep(from, to, [&](uint32_t k, int) {
             const uint32_t d = (k >> shift) & mask;
             atomicAdd(&sh.cnt[d], 1u);
             if (by_mass) {
@@ -369,18 +385,49 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
             }
         });
         cluster_sync();
-        // this block's slice, the highest digit first
+        // this block's slice, added up over the cluster: a thread reads four neighbouring digits of one block (eight neighbouring
+        // lanes: the same digits of the eight blocks), so that everything is on its way at once
+        {
+            const int quad = tid >> 3, q = tid & 7;
+            const uint32_t d0 = me * SLICE + 4 * quad;
+            uint4 cv = *peer(reinterpret_cast<uint4*>(&sh.cnt[d0]), q);
+            unsigned long long mv[4] = {0, 0, 0, 0};
+            if (by_mass) {
+                if (STAGED) {
+                    const uint4 a = *peer(reinterpret_cast<uint4*>(&sh.mass[0][d0]), q), b = *peer(reinterpret_cast<uint4*>(&sh.mass[1][d0]), q),
+                                c = *peer(reinterpret_cast<uint4*>(&sh.mass[2][d0]), q);
+                    mv[0] = a.x + ((unsigned long long)b.x << 14) + ((unsigned long long)c.x << 28);
+                    mv[1] = a.y + ((unsigned long long)b.y << 14) + ((unsigned long long)c.y << 28);
+                    mv[2] = a.z + ((unsigned long long)b.z << 14) + ((unsigned long long)c.z << 28);
+                    mv[3] = a.w + ((unsigned long long)b.w << 14) + ((unsigned long long)c.w << 28);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) mv[e] = *peer(&sh.whole_mass[d0 + e], q);
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                cv.x += __shfl_xor_sync(0xffffffffu, cv.x, o);
+                cv.y += __shfl_xor_sync(0xffffffffu, cv.y, o);
+                cv.z += __shfl_xor_sync(0xffffffffu, cv.z, o);
+                cv.w += __shfl_xor_sync(0xffffffffu, cv.w, o);
+                if (by_mass)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) mv[e] += __shfl_xor_sync(0xffffffffu, mv[e], o);
+            }
+            if (q == 0) {
+                *reinterpret_cast<uint4*>(&sh.slice_cnt[4 * quad]) = cv;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sh.slice_mass[4 * quad + e] = mv[e];
+            }
+            __syncthreads();
+        }
+        // the highest digit first
         const uint32_t d = me * SLICE + SLICE - 1 - tid;
         unsigned long long c = 0, m = 0;
         if (tid < SLICE) {
-#pragma unroll
-            for (int q = 0; q < SC; ++q) {
-                c += *peer(&sh.cnt[d], q);
-                if (by_mass)
-                    m += STAGED ? *peer(&sh.mass[0][d], q) + ((unsigned long long)*peer(&sh.mass[1][d], q) << 14) +
-                                      ((unsigned long long)*peer(&sh.mass[2][d], q) << 28)
-                                : *peer(&sh.whole_mass[d], q);
-            }
+            c = sh.slice_cnt[SLICE - 1 - tid];
+            m = sh.slice_mass[SLICE - 1 - tid];
             if (by_mass && extra && (extra_key >> shift >> bits) == prefix && d == ((extra_key >> shift) & mask)) {
                 c += extra;
                 m += extra_mass;
@@ -428,9 +475,10 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
     uint32_t kth_key = 0;
     unsigned int ties_k = UINT_MAX;
     if (top_k > 0 && top_k < V) {
-        // At least top_k elements reach the top_k-th largest of the warps' maxima: what is below it need not be counted.
+        // At least top_k elements reach the top_k-th largest of the warps' maxima: what is below it is out.
         uint32_t floor_key = 0;
         if (top_k <= SC * SWARPS) {
+            if (tid == 0) sh.n_own = 0;
             if (tid < SC * SWARPS) {
                 const uint32_t v = sh.peer_warp_max[tid];
                 int greater = 0, reach = 0;
@@ -442,6 +490,65 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
             }
             __syncthreads();
             floor_key = sh.floor_key;
+            // The short way: what is left is usually little more than top_k elements of the whole row.  Block 0 gets them all
+            // and finishes alone, on lists, with one exchange instead of twenty.
+            sweep(floor_key, UINT_MAX, [&](uint32_t k, int i) {
+                const uint32_t at = atomicAdd(&sh.n_own, 1u);
+                if (at < CAP) sh.list.own[at] = make_uint2(k, (uint32_t)(lo + i));
+            });
+            __syncthreads();
+            const uint32_t n_own = sh.n_own;
+            if (tid < min(n_own, (uint32_t)CAP)) *peer(&sh.list.all[me][tid], 0) = sh.list.own[tid];
+            if (tid < SC) *peer(&sh.peer_found[me], tid) = n_own;
+            cluster_sync();
+            uint32_t found = 0, most = 0;
+#pragma unroll
+            for (int q = 0; q < SC; ++q) {
+                found += sh.peer_found[q];
+                most = max(most, sh.peer_found[q]);
+            }
+            if (most <= CAP && found <= ST) {
+                if (me != 0) return;                                              // (nothing of this block is read any more)
+                int mine = -1;                                                    // thread t has the t-th of all lists, one after the other
+                uint2 cand = make_uint2(0, 0);
+                for (int q = 0, first = 0; q < SC; first += sh.peer_found[q], ++q)
+                    if (tid >= first && tid < first + (int)sh.peer_found[q]) { mine = tid; cand = sh.list.all[q][tid - first]; }
+                // its place by key (the first of equals first) and by index
+                int by_key = 0, by_index = 0;
+                if (mine >= 0)
+                    for (int q = 0; q < SC; ++q)
+                        for (uint32_t j = 0; j < sh.peer_found[q]; ++j) {
+                            const uint2 o = sh.list.all[q][j];
+                            by_key += o.x > cand.x || (o.x == cand.x && o.y < cand.y);
+                            by_index += o.y < cand.y;
+                        }
+                const unsigned long long m = mine >= 0 && by_key < top_k ? mass_fp(key_value(cand.x), mx, inv_t) : 0;
+                if (mine >= 0) sh.list.by_key[by_key] = m;
+                __syncthreads();
+                unsigned long long zk, before;
+                before = block_excl_scan(tid < (int)found ? sh.list.by_key[tid] : 0, sh.scan, &zk);
+                unsigned long long reach = (unsigned long long)ceil((double)top_p * (double)zk);
+                if (reach < 1) reach = 1;
+                sh.list.kept[tid] = tid < top_k && (top_p >= 1.0f || before < reach);
+                __syncthreads();
+                if (mine >= 0) {
+                    sh.list.by_index[by_index] = sh.list.kept[by_key] ? m : 0;
+                    sh.list.index[by_index] = (int)cand.y;
+                }
+                __syncthreads();
+                const unsigned long long own = tid < (int)found ? sh.list.by_index[tid] : 0;
+                unsigned long long total;
+                before = block_excl_scan(own, sh.scan, &total);
+                if (total == 0) {
+                    if (tid == 0) out[r] = top.i;
+                    return;
+                }
+                const double u = llb_uniform(seed, (unsigned long long)(keys ? keys[r] : r), (unsigned long long)(steps ? steps[r] : 0));
+                unsigned long long at = (unsigned long long)(u * (double)total);
+                if (at >= total) at = total - 1;
+                if (at >= before && at < before + own) out[r] = sh.list.index[tid];
+                return;
+            }
         }
         uint32_t prefix = 0, rem = (uint32_t)top_k;
 #pragma unroll 1
@@ -460,12 +567,12 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
     if (top_p < 1.0f) {
         const unsigned long long kth_mass = mass_fp(key_value(kth_key), mx, inv_t);
         unsigned long long part = 0, own, equal = 0;
-        if (kth_key < UINT_MAX) sweep(kth_key + 1, UINT_MAX, [&](uint32_t k) { part += mass_fp(key_value(k), mx, inv_t); });
+        if (kth_key < UINT_MAX) sweep(kth_key + 1, UINT_MAX, [&](uint32_t k, int) { part += mass_fp(key_value(k), mx, inv_t); });
         block_excl_scan(part, sh.scan, &own);
         unsigned long long zk = cluster_sum(0, own, nullptr);
         unsigned int n_eq_kept = ties_k;
         if (ties_k == UINT_MAX) {             // no top-k: every element equal to the minimum key counts
-            sweep(kth_key, kth_key, [&](uint32_t) { ++equal; });
+            sweep(kth_key, kth_key, [&](uint32_t, int) { ++equal; });
             block_excl_scan(equal, sh.scan, &own);
             n_eq_kept = (unsigned)cluster_sum(1, own, nullptr);
         }
