@@ -39,11 +39,17 @@
 // (cp.reduce.async.bulk.tensor ... add) per 32 tokens from a float32 staging buffer.  Nothing is
 // gathered or re-read: the sums meet in the L2.
 //
+// MOE (instantiations of their own): the same pairs over the tiles of a routed step's plan (csrc/moe.cu): a tile is 256 rows of one
+// expert's matrix x up to 256 of the slots that chose it.  1: the product, plain or through the expert's activation, stored in
+// slot order; 2: every slot's row times the slot's weight, added to its token's row of the float32 stream (float32 atomics).
+// The number of tiles is known on the device only.
+//
 // Every wait on an mbarrier is bounded; when a bound is hit the role records an error code in
 // *err and stops, the other roles run into their own bounds, and both CTAs meet at the final
 // cluster barrier, free their tensor memory and return.
 #include "common.cuh"
 #include "tma_map.cuh"
+#include <limits.h>
 
 namespace {
 
@@ -169,6 +175,13 @@ struct Gemm2Args {
     int* err;
     int ksplit, chunk_kb;  // INTO: K ranges per tile and k-blocks per range (1 and all of them otherwise)
     GluForm glu = {};      // DUAL: how gate and up combine
+    // MOE: the plan's tiles [3, max_tiles] (expert, first slot, slots) and their number; rows_out is a matrix's rows
+    const int* moe_tiles = nullptr;
+    const int* moe_n = nullptr;
+    int moe_max = 0, moe_act = 0, moe_top = 1;
+    const int* pair_of = nullptr;      // MOE 2: slot -> pair (token * top + choice)
+    const float* wgt = nullptr;        //        pair -> weight
+    float* sum = nullptr;              //        the stream [T, ldy]
 
     // Tile t's block of weight rows and its block of tokens.  Tiles are walked in bands of `group` weight blocks: inside a band the
     // weight block changes first, then the token block, so that the tiles which the pairs work on at one time form a
@@ -178,6 +191,25 @@ struct Gemm2Args {
         const int rows = min(group, row_tiles - band * group);
         tok_tile = in_band / rows;
         row_tile = band * group + in_band - tok_tile * rows;
+    }
+    // Unit u's first weight row in W (`rank`'s half of the pair's tile), its first output column, its first token or slot, and the
+    // end of its tokens or slots.  MOE: a tile's blocks of rows follow one another, so that its slots are met at one time.
+    template <int MOE>
+    __device__ __forceinline__ void unit(int u, int rank, int mrows, int bn, int& w_row, int& m0, int& n0, int& n_end) const {
+        int row_tile, tok_tile;
+        if (MOE) {
+            tok_tile = u / row_tiles;
+            row_tile = u - tok_tile * row_tiles;
+            m0 = (row_tile * 2 + rank) * mrows;
+            w_row = moe_tiles[tok_tile] * rows_out + m0;
+            n0 = moe_tiles[moe_max + tok_tile];
+            n_end = n0 + moe_tiles[2 * moe_max + tok_tile];
+        } else {
+            place(u % n_tiles, row_tile, tok_tile);
+            w_row = m0 = (row_tile * 2 + rank) * mrows;
+            n0 = tok_tile * bn;
+            n_end = T;
+        }
     }
 };
 
@@ -214,7 +246,7 @@ struct Smem2 {
     static_assert(TOTAL <= 232448, "a block's shared memory");
 };
 
-template <int BN, int STAGES, int DUAL, bool INTO = false>
+template <int BN, int STAGES, int DUAL, bool INTO = false, int MOE = 0>
 __global__ void __launch_bounds__(THREADS)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                 const __grid_constant__ CUtensorMap map_out, Gemm2Args g) {
@@ -237,7 +269,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int pair = blockIdx.x >> 1;
     const int kblocks = (g.K + BK - 1) / BK;
     // work units: unit u is tile u % n_tiles over the k-blocks [(u / n_tiles) * chunk_kb, ...) (one unit per tile unless INTO)
-    const int n_units = g.n_tiles * g.ksplit;
+    int n_units = g.n_tiles * g.ksplit;
     auto unit_kb0 = [&](int u) { return (u / g.n_tiles) * g.chunk_kb; };
     auto unit_kb1 = [&](int u) { return min(kblocks, (u / g.n_tiles + 1) * g.chunk_kb); };
 
@@ -268,13 +300,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
     // The weight does not depend on any earlier kernel of the step: the first tile's first STAGES k-blocks of it are
     // requested before the grid dependency resolves, while the predecessor is still running.
-    const int first_kb0 = unit_kb0(pair);
-    const int prefetched = min(STAGES, unit_kb1(pair) - first_kb0);
-    if (warp == 0 && lane == 0) {
+    // (MOE: which weight is known behind it only)
+    const int first_kb0 = MOE ? 0 : unit_kb0(pair);
+    const int prefetched = MOE ? 0 : min(STAGES, unit_kb1(pair) - first_kb0);
+    if (!MOE && warp == 0 && lane == 0) {
         const uint32_t full0 = mapa(bar_full, 0);
-        int row_tile, tok_tile;
-        g.place(pair % g.n_tiles, row_tile, tok_tile);
-        const int m0 = (row_tile * 2 + (int)rank) * MROWS;
+        int w_row, m0, n0, n_end;
+        g.template unit<0>(pair, (int)rank, MROWS, BN, w_row, m0, n0, n_end);
         for (int i = 0; i < prefetched; ++i) {
             const uint32_t dst = base + i * S::STAGE_BYTES, bar = full0 + 8 * i;
             if (leader) mbar_expect_tx(bar_full + 8 * i, 2u * S::STAGE_BYTES);
@@ -283,15 +315,16 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
     }
     llb_grid_dependency_sync();      // from here on memory written by earlier kernels is touched
+    if (MOE) n_units = *g.moe_n * g.row_tiles;
 
     if (warp == 0) {
         // ---- producer: this CTA's weight rows and its half of the tokens, k-block after k-block, tile after tile.  The
         // warp waits for a free stage as a whole; one elected lane issues the copies.
         const uint32_t full0 = mapa(bar_full, 0);
-        if (elect_one()) {   // the activations of the k-blocks whose weight is on its way already
-            int row_tile, tok_tile;
-            g.place(pair % g.n_tiles, row_tile, tok_tile);
-            const int n0 = tok_tile * BN + (int)rank * (BN / 2);
+        if (!MOE && elect_one()) {   // the activations of the k-blocks whose weight is on its way already
+            int w_row, m0, n0, n_end;
+            g.template unit<0>(pair, (int)rank, MROWS, BN, w_row, m0, n0, n_end);
+            n0 += (int)rank * (BN / 2);
             for (int i = 0; i < prefetched; ++i)
                 tma_load_2d_pair(base + i * S::STAGE_BYTES + ACCS * S::A_BYTES, &map_x, full0 + 8 * i, (first_kb0 + i) * BK, n0, g.hint_x);
         }
@@ -299,12 +332,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         int it = prefetched;
         bool ok = true;
         for (int u = pair; u < n_units && ok; u += g.n_pairs) {
-            const int kb1 = unit_kb1(u);
-            int row_tile, tok_tile;
-            g.place(u % g.n_tiles, row_tile, tok_tile);
-            const int m0 = (row_tile * 2 + (int)rank) * MROWS;
-            const int n0 = tok_tile * BN + (int)rank * (BN / 2);
-            for (int kb = unit_kb0(u) + (u == pair ? prefetched : 0); kb < kb1; ++kb, ++it) {
+            const int kb1 = MOE ? kblocks : unit_kb1(u);
+            int w_row, m0, n0, n_end;
+            g.template unit<MOE>(u, (int)rank, MROWS, BN, w_row, m0, n0, n_end);
+            n0 += (int)rank * (BN / 2);
+            for (int kb = (MOE ? 0 : unit_kb0(u)) + (u == pair ? prefetched : 0); kb < kb1; ++kb, ++it) {
                 const int s = it % STAGES;
                 if (it >= STAGES && !warp_wait(bar_empty + 8 * s, (uint32_t)(it / STAGES - 1) & 1u, &s_abort)) {
                     if (lane == 0 && !s_abort) { s_abort = 1; atomicExch(g.err, ERR_TC2_WAIT_EMPTY); }
@@ -314,7 +346,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (elect_one()) {
                     const uint32_t dst = base + s * S::STAGE_BYTES, bar = full0 + 8 * s;
                     if (leader) mbar_expect_tx(bar_full + 8 * s, 2u * S::STAGE_BYTES);
-                    tma_load_2d_pair(dst, &map_w, bar, kb * BK, m0, g.hint_w);
+                    tma_load_2d_pair(dst, &map_w, bar, kb * BK, w_row, g.hint_w);
                     if (DUAL) tma_load_2d_pair(dst + S::A_BYTES / (3 - DUAL), &map_w, bar, kb * BK, m0 + g.dual_offset, g.hint_w);
                     tma_load_2d_pair(dst + ACCS * S::A_BYTES, &map_x, bar, kb * BK, n0, g.hint_x);
                 }
@@ -337,7 +369,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             int it = 0, ti = 0;
             bool ok = true;
             for (int u = pair; u < n_units && ok; u += g.n_pairs, ++ti) {
-                const int buf = ti % NBUF, kb0 = unit_kb0(u), kb1 = unit_kb1(u);
+                const int buf = ti % NBUF, kb0 = MOE ? 0 : unit_kb0(u), kb1 = MOE ? kblocks : unit_kb1(u);
                 if (ti >= NBUF && !warp_wait(bar_acc_empty + 8 * buf, (uint32_t)(ti / NBUF - 1) & 1u, &s_abort)) {
                     if (lane == 0 && !s_abort) { s_abort = 1; atomicExch(g.err, ERR_TC2_WAIT_ACC_EMPTY); }
                     break;
@@ -393,13 +425,20 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         int ti = 0, chunk_i = 0;
         for (int u = pair; u < n_units; u += g.n_pairs, ++ti) {
             const int buf = ti % NBUF;
-            int row_tile, tok_tile;
-            g.place(u % g.n_tiles, row_tile, tok_tile);
-            const int m0 = (row_tile * 2 + (int)rank) * MROWS;
-            const int n0 = tok_tile * BN;
+            int w_row, m0, n0, n_end;
+            g.template unit<MOE>(u, (int)rank, MROWS, BN, w_row, m0, n0, n_end);
             const int m = m0 + row;
+            // MOE 2: lane l has token and weight of the slots that the warp meets as its l-th and its (l + 32)-th
+            int tok_a = 0, tok_b = 0;
+            float wgt_a = 0.f, wgt_b = 0.f;
+            if (MOE == 2) {
+                static_assert(BN / CHUNK * COLS == 64 || MOE != 2, "a warp meets 64 slots of a tile");
+                const int sa = n0 + (lane / COLS) * CHUNK + h + lane % COLS, sb = sa + 32 / COLS * CHUNK;
+                if (sa < n_end) { const int pr = g.pair_of[sa]; tok_a = pr / g.moe_top; wgt_a = g.wgt[pr]; }
+                if (sb < n_end) { const int pr = g.pair_of[sb]; tok_b = pr / g.moe_top; wgt_b = g.wgt[pr]; }
+            }
             float bias_v = 0.f;
-            if (!DUAL && g.bias && m < g.rows_out && u < g.n_tiles)    // the bias goes in with the first K range only
+            if (!DUAL && !MOE && g.bias && m < g.rows_out && u < g.n_tiles)    // the bias goes in with the first K range only
                 bias_v = g.bias_dtype == LLB_F32 ? ((const float*)g.bias)[m] : to_f32(((const bf16*)g.bias)[m]);
             if (!mbar_wait(bar_acc_full + 8 * buf, (uint32_t)(ti / NBUF) & 1u, &s_abort)) {
                 s_epi_abort = 1;
@@ -414,8 +453,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             uint32_t nxt0[COLS], nxt1[COLS];
             tmem_ld_cols_nowait(acc + h, nxt0);
             if (DUAL == 2) tmem_ld_cols_nowait(acc + BN + h, nxt1);
+            const int c_end = MOE ? min(BN, n_end - n0) : BN;      // (columns behind a tile's last slot are not read)
 #pragma unroll 1
-            for (int c = 0; c < BN; c += CHUNK, ++chunk_i) {
+            for (int c = 0; c < c_end; c += CHUNK, ++chunk_i) {
                 float v0[COLS], v1[COLS];
                 tmem_wait_ld_cols(nxt0);
                 if (DUAL == 2) pin_cols(nxt1);                     // (loaded before the wait: valid behind it)
@@ -424,9 +464,28 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     v0[j] = __uint_as_float(nxt0[j]);
                     if (DUAL == 2) v1[j] = __uint_as_float(nxt1[j]);
                 }
-                if (c + CHUNK < BN) {
+                if (c + CHUNK < c_end) {
                     tmem_ld_cols_nowait(acc + c + CHUNK + h, nxt0);
                     if (DUAL == 2) tmem_ld_cols_nowait(acc + BN + c + CHUNK + h, nxt1);
+                }
+                if (MOE == 2) {
+                    // 32 neighbouring columns of a token's row a warp instruction: whole 128-byte lines of atomics
+                    const int at = (c / CHUNK) * COLS;             // the chunk's first slot in the warp's order
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j) {
+                        const int from = (at + j) & 31;
+                        const int tok = __shfl_sync(0xffffffffu, at < 32 ? tok_a : tok_b, from);
+                        const float wv = __shfl_sync(0xffffffffu, at < 32 ? wgt_a : wgt_b, from);
+                        if (m < g.rows_out && n0 + c + h + j < n_end) atomicAdd(g.sum + (size_t)tok * g.ldy + m, wv * v0[j]);
+                    }
+                    continue;
+                }
+                if (MOE == 1) {
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j) {
+                        if (g.moe_act == 1) { v0[j] = fmaxf(v0[j], 0.f); v0[j] *= v0[j]; }
+                        if (g.moe_act == 3) v0[j] = 0.5f * v0[j] * (1.0f + erff(v0[j] * 0.7071067811865476f));
+                    }
                 }
                 if (INTO) {
                     // this K range's partial sums of 32 tokens x 128 rows, laid out as they lie in the stream, then one
@@ -485,7 +544,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
                     for (int j = lane >> 2; j < COLS; j += 8) {
                         const int n = n0 + c + h + j;
-                        if (n < g.T)
+                        if (n < n_end)
                             *reinterpret_cast<uint4*>(g.Y + (size_t)n * g.ldy + mcol) =
                                 *reinterpret_cast<const uint4*>(sw + j * 32 + piece * 8);
                     }
@@ -513,9 +572,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-template <int BN, int STAGES, int DUAL, bool INTO = false>
+template <int BN, int STAGES, int DUAL, bool INTO = false, int MOE = 0>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, const Gemm2Args& g, cudaStream_t stream) {
-    auto k = gemm_tc2_kernel<BN, STAGES, DUAL, INTO>;
+    auto k = gemm_tc2_kernel<BN, STAGES, DUAL, INTO, MOE>;
     constexpr int smem = Smem2<BN, STAGES, DUAL, INTO>::TOTAL;
     static bool configured[64] = {};         // function attributes belong to a device's copy of the kernel
     int dev = 0;
@@ -664,4 +723,41 @@ LLB_API int llb_gemm_tc2_into(const void* X, const void* W, const void* bias, in
     rc = llb_tma::f32_map_plain(stream_, T, N, lds, BM, CHUNK, &mo);
     if (rc) return rc;
     return launch<256, 6, 0, true>(mw, mx, mo, g, stream);
+}
+
+// The experts' products of a routed step whose plan has tiles of 256 slots: A [slots, K] bf16 (row stride lda) in slot order, W [E, N, K]
+// bf16 dense.  epilogue 0, 1 and 3: out [slots, ldo] bf16 = the product, its squared ReLU, its gelu (erf form); 2: out is
+// the float32 stream [T, ldo], and row token(slot) gets weight(slot) * product added.  K, lda, and N and ldo of a stored
+// result, are multiples of 8, all bases 16-byte aligned.  The grid covers the device; pairs without a tile leave at once.
+LLB_API int llb_moe_gemm_tc2(const void* A, int lda, long long n_slots, const void* W, int E, int N, int K, void* out, int ldo,
+                             const int* tiles, int max_tiles, const int* n_tiles, int epilogue, const int* pair_of, const float* wgt,
+                             int top, int max_pairs, int* err, cudaStream_t stream) {
+    if (max_tiles == 0 || N == 0 || n_slots == 0) return 0;
+    const bool add = epilogue == 2;
+    if (K <= 0 || K % 8 || lda % 8 || max_pairs < 1 || epilogue < 0 || epilogue > 3 || (!add && (N % 8 || ldo % 8)) ||
+        (add && (!pair_of || !wgt || top < 1)) || (((uintptr_t)A | (uintptr_t)W) & 15) || ((uintptr_t)out & (add ? 3 : 15)) || (long long)E * N > INT_MAX || n_slots > INT_MAX)
+        return (int)cudaErrorInvalidValue;
+    Gemm2Args g;
+    g.bias = nullptr; g.bias_dtype = 0; g.Y = (bf16*)out; g.sum = (float*)out;
+    g.T = (int)n_slots; g.K = K; g.ldy = ldo; g.rows_out = N; g.dual_offset = 0;
+    g.tok_tiles = max_tiles;
+    const int row_tiles = (N + 2 * BM - 1) / (2 * BM);
+    if ((long long)row_tiles * max_tiles > (1 << 30)) return (int)cudaErrorInvalidValue;
+    g.row_tiles = row_tiles;
+    g.group = 1;
+    g.hint_w = HINT_EVICT_FIRST;                 // an expert's matrix is read once where one tile holds its slots
+    g.hint_x = HINT_EVICT_LAST;
+    g.n_tiles = row_tiles * max_tiles;
+    g.n_pairs = g.n_tiles < max_pairs ? g.n_tiles : max_pairs;
+    g.err = err;
+    g.ksplit = 1;
+    g.chunk_kb = (K + BK - 1) / BK;
+    g.moe_tiles = tiles; g.moe_n = n_tiles; g.moe_max = max_tiles; g.moe_act = epilogue; g.moe_top = top;
+    g.pair_of = pair_of; g.wgt = wgt;
+    CUtensorMap mw, mx;
+    int rc = llb_tma::bf16_map_64(W, (long long)E * N, K, K, BM, &mw);
+    if (rc) return rc;
+    rc = llb_tma::bf16_map_64(A, n_slots, K, lda, 128, &mx);
+    if (rc) return rc;
+    return add ? launch<256, 6, 0, false, 2>(mw, mx, mw, g, stream) : launch<256, 6, 0, false, 1>(mw, mx, mw, g, stream);
 }

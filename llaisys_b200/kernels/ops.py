@@ -1201,10 +1201,13 @@ def moe_tc_ok(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor) -> bool:
 
 
 def moe_tc_tile_rows(n_pairs: int, n_experts: int) -> int:
-    """Slots of a tile of the tensor-core product: 16, 64 or 128 by the pairs an expert gets on average (a function of
-    the step's shape alone)."""
+    """Slots of a tile of the tensor-core product: 16, 64 or 256 by the pairs an expert gets on average (a function of
+    the step's shape alone).  Tiles of 256 run on pairs of SMs (csrc/gemm_tc2.cu): an expert's matrix is then read once, which is what
+    such a step cannot do without.  Up and down of 64 experts, 6 a token, 2,048 <-> 1,408, us with tiles of 64 / 128 / 256:
+    145 / 150 / 150 at 38 pairs an expert, 152 / 157 / 150 at 48, 168 / 166 / 153 at 66, 200 / 184 / 156 at 96, 320 / 274 / 172 at
+    192, 684 / 564 / 321 at 469."""
     avg = n_pairs / max(1, n_experts)
-    return 16 if avg <= 16 else 64 if avg <= 96 else 128
+    return 16 if avg <= 16 else 64 if avg <= 48 else 256
 
 
 def moe_gather_rows(x: torch.Tensor, plan: MoePlan) -> torch.Tensor:
@@ -1226,13 +1229,22 @@ def moe_gemm_tc(a: torch.Tensor, w: torch.Tensor, plan: MoePlan, epilogue: str, 
     _need_cuda(a, w, out, wgt)
     E, N, K = w.shape
     assert w.is_contiguous() and a.stride(1) == 1 and a.shape == (plan.n_pairs, K) and a.dtype == w.dtype == torch.bfloat16
-    assert plan.max_tiles and plan.tile_rows in (16, 64, 128)
+    assert plan.max_tiles and plan.tile_rows in (16, 64, 256)
     code = {"store": 0, "relu_squared": 1, "weighted_add": 2, "gelu": 3}[epilogue]
     if code == 2:
         assert out is not None and out.dtype == torch.float32 and out.stride(1) == 1 and out.shape[1] == N and wgt is not None
     else:
         out = torch.empty((plan.n_pairs, N), dtype=out_dtype, device=a.device)
     err = _tc_resources(a.device)[2]
+    if plan.tile_rows == 256:
+        assert code == 2 or out.dtype == torch.bfloat16
+        f = _fn(_stamped("gemm_tc2.cu"), "llb_moe_gemm_tc2",
+                [c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
+                 c_void_p, c_int, c_int, c_void_p, c_void_p])
+        _check(f(_ptr(a), a.stride(0), plan.n_pairs, _ptr(w), E, N, K, _ptr(out), out.stride(0), _ptr(plan.tiles), plan.max_tiles,
+                 _ptr(plan.n_tiles), code, _ptr(plan.pair_of), _ptr(wgt), plan.top, _sm_count(a.device) // 2, _ptr(err), _stream()),
+               "experts' product (tensor cores, paired SMs)")
+        return out
     f = _fn(load_module("moe_tc.cu"), "llb_moe_gemm_tc",
             [c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int,
              c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p])

@@ -671,6 +671,39 @@ def test_feed_forward_in_one_launch(T, H, I, stages):
     assert float((two - res).abs().max()) <= 2.0 ** -7 * float((res - res0).abs().max()) + 1e-3
 
 
+@pytest.mark.parametrize("T,E,top,H,ff,skew", [(40, 1, 1, 64, 8, 1.0), (257, 1, 1, 72, 264, 1.0), (300, 2, 2, 128, 256, 1.0), (700, 5, 3, 200, 520, 3.0),
+                                               (1500, 16, 2, 512, 136, 1.5), (512, 3, 1, 64, 1408, 9.0)])
+def test_experts_products_in_tiles_of_256_slots(T, E, top, H, ff, skew):
+    """The products on pairs of SMs over a plan's tiles: experts with one slot, exactly a tile's, several tiles and none, row blocks that
+    end inside an expert's matrix (the next expert's rows are computed beside it and not stored), every activation."""
+    from llaisys_b200 import kernels
+    gen = torch.Generator(device=DEV).manual_seed(T + E)
+    p = torch.rand(T, E, device=DEV, generator=gen) ** skew * torch.arange(E, device=DEV).clamp_max(3)      # expert 0: none, unless needed
+    idx = p.topk(top, -1).indices.int()
+    wgt = torch.rand(T, top, device=DEV, generator=gen) + 0.5
+    x = torch.randn(T, H, device=DEV, generator=gen).bfloat16()
+    up = (torch.randn(E, ff, H, device=DEV, generator=gen) * H ** -0.5).bfloat16()
+    down = (torch.randn(E, H, ff, device=DEV, generator=gen) * ff ** -0.5).bfloat16()
+    plan = kernels.moe_plan(idx, E, 256)
+    rows = kernels.moe_gather_rows(x, plan)
+    pair = plan.pair_of.long()
+    slot_e, tok, w = idx.reshape(-1)[pair].long(), pair // top, wgt.reshape(-1)[pair].double()
+    pre = torch.einsum("sk,snk->sn", x[tok].double(), up.double()[slot_e]) if T * top * ff * H < 5e7 else torch.stack(
+        [x[t].double() @ up[e].double().T for t, e in zip(tok.tolist(), slot_e.tolist())])
+    wants = {"store": pre, "relu_squared": pre.clamp_min(0) ** 2, "gelu": torch.nn.functional.gelu(pre)}
+    for act, want in wants.items():
+        got = kernels.moe_gemm_tc(rows, up, plan, act)
+        assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * math.sqrt(H)).all()), act
+    got = kernels.moe_gemm_tc(rows, up, plan, "store")
+    want = torch.zeros(T, H, device=DEV, dtype=torch.float64)
+    y = torch.stack([got[i].double() @ down[e].double().T for i, e in enumerate(slot_e.tolist())])
+    want.index_add_(0, tok, w[:, None] * y)
+    stream = torch.ones(T, H, device=DEV)
+    kernels.moe_gemm_tc(got, down, plan, "weighted_add", out=stream, wgt=wgt)
+    assert float((stream.double() - 1 - want).abs().max()) <= 1e-5 * math.sqrt(ff) * (1 + float(want.abs().max()))
+    assert kernels.tc_error(DEV) == 0
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_random_weights_are_the_same_numbers_on_the_device_and_on_the_host(dtype):
     """The device kernel and its numpy twin perform the same IEEE operations in the same order: a tensor made on
