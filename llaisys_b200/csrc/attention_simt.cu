@@ -48,6 +48,19 @@ constexpr int ROWS = (DH <= 256 || ROWS32_FIT) ? 32 : 8;
 constexpr int WARPS = 4;
 constexpr int RPW = ROWS / WARPS;   // rows of a warp
 constexpr int DPL = (DV + 31) / 32; // output dims of a lane
+// The usual head sizes: a warp takes its eight rows through a tile together, so that a key or a value that it reads from shared memory (16
+// bytes a lane) serves all of them.  Row by row, element by element, every FMA had 1.5 reads of its own and the SM's shared
+// memory was what a tile waited for.  (256 tokens, 12 heads of 128, float32: prefill 110 -> 64 us a layer.)
+constexpr bool TOGETHER = RPW == 8 && DH % 4 == 0 && DH <= 256 && (DV == 32 || DV == 64 || DV == 128 || DV == 256);
+constexpr int KP = TOGETHER ? DH + 4 : DH + 1;       // floats from one key row of a tile to the next: neighbouring rows in other banks
+constexpr int PS = TOGETHER ? RPW : 1;               // rows whose probabilities a warp keeps at one time
+constexpr int VW = DV / 32 < 1 ? 1 : DV / 32 > 4 ? 4 : DV / 32;     // TOGETHER: neighbouring output dims of a lane
+// the e-th output dim of a lane
+__device__ __forceinline__ int out_dim(int lane, int e) { return TOGETHER ? (e / VW) * (32 * VW) + lane * VW + e % VW : lane + e * 32; }
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ float halves_sum(f32x2 v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
 
 struct AttnParams {
     const void* q;        // packed projections [T, row_stride]; query head h at column h * DH
@@ -99,10 +112,10 @@ template <typename T, bool DECODE>
 __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
     extern __shared__ float smem[];
     float* Qs = smem;                        // [ROWS][DH]
-    float* Ks = Qs + ROWS * DH;              // [LLB_PAGE][DH + 1]
-    float* Vs = Ks + LLB_PAGE * (DH + 1);    // [LLB_PAGE][DV]; with v_in_k the key tile itself
-    float* Ps = Vs + (p.v_in_k ? 0 : LLB_PAGE * DV);   // [WARPS][LLB_PAGE]
-    const int vs_stride = p.v_in_k ? DH + 1 : DV;
+    float* Ks = Qs + ROWS * DH;              // [LLB_PAGE][KP]
+    float* Vs = Ks + LLB_PAGE * KP;          // [LLB_PAGE][DV]; with v_in_k the key tile itself
+    float* Ps = Vs + (p.v_in_k ? 0 : LLB_PAGE * DV);   // [WARPS][LLB_PAGE][PS]
+    const int vs_stride = p.v_in_k ? KP : DV;
     if (p.v_in_k) Vs = Ks;
     const int kv_stride = p.kv_row_stride > 0 ? p.kv_row_stride : p.row_stride;
 
@@ -191,7 +204,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             const T* vp = (const T*)p.pool_v + paged_row(ptab, p.pool_table_stride, p0, vh, cache_heads, DV, 0);
             for (int i = tid; i < LLB_PAGE * DH; i += WARPS * 32) {
                 const int j = i / DH, d = i - j * DH;
-                Ks[j * (DH + 1) + d] = p0 + j < blocks_hi ? to_f32(kp[(size_t)j * krow + d]) : 0.f;
+                Ks[j * KP + d] = p0 + j < blocks_hi ? to_f32(kp[(size_t)j * krow + d]) : 0.f;
             }
             for (int i = tid; i < LLB_PAGE * DV; i += WARPS * 32) {
                 const int j = i / DV, d = i - j * DV;
@@ -228,7 +241,13 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
                     for (int u = 0; u < BATCH; ++u) {
                         const int i = i0 + u * WARPS * 32, j = i / PER, d = (i - j * PER) * VEC;
                         const T* rv = reinterpret_cast<const T*>(&raw[u]);
-                        if (i < PIECES)
+                        if (i >= PIECES) continue;
+                        if (pitch % 4 == 0)
+#pragma unroll
+                            for (int e = 0; e < VEC; e += 4)
+                                *reinterpret_cast<float4*>(dst + j * pitch + d + e) =
+                                    make_float4(to_f32(rv[e]), to_f32(rv[e + 1]), to_f32(rv[e + 2]), to_f32(rv[e + 3]));
+                        else
 #pragma unroll
                             for (int e = 0; e < VEC; ++e) dst[j * pitch + d + e] = to_f32(rv[e]);
                     }
@@ -242,14 +261,52 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             }
         };
         if (!pooled) {
-            fetch_tile(IntC<DH>(), Ks, DH + 1, kpool, kpage, krow, knew, kvh * DH);
+            fetch_tile(IntC<DH>(), Ks, KP, kpool, kpage, krow, knew, kvh * DH);
             if (!p.v_in_k)
                 fetch_tile(IntC<DV>(), Vs, DV, vpool, cached ? vpool + paged_row(table, p.ring, p0, vh, cache_heads, DV, p.pinned) : nullptr, DV,
                            vnew, vh * DV);
         }
         __syncthreads();
+        const int my_rows = n_rows > warp ? (n_rows - warp + WARPS - 1) / WARPS : 0;      // rows warp, warp + WARPS, ... of the block
+        float* ps = Ps + warp * LLB_PAGE * PS;
+        // both keys' scores of all rows (each as an even and an odd half: fma.rn.f32x2 is two float32 FMAs)
+        float dot[TOGETHER ? RPW : 1][2];
+        if constexpr (TOGETHER) {
+            // (rows beyond the block's own compute on whatever lies there and are not used)
+            auto dots = [&](auto rows) {
+                constexpr int N = decltype(rows)::value;
+                f32x2 acc[N][2];
+#pragma unroll
+                for (int i = 0; i < N; ++i) acc[i][0] = acc[i][1] = 0;
+                const float* k0 = Ks + lane * KP;
+                const float* k1 = Ks + (lane + 32) * KP;
+                const float* q0 = Qs + warp * DH;
+#pragma unroll 4
+                for (int d = 0; d < DH; d += 4) {
+                    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(k0 + d), c = *reinterpret_cast<const ulonglong2*>(k1 + d);
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(q0 + i * WARPS * DH + d);
+                        fma2(acc[i][0], q.x, a.x);
+                        fma2(acc[i][1], q.x, c.x);
+                        fma2(acc[i][0], q.y, a.y);
+                        fma2(acc[i][1], q.y, c.y);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    dot[i][0] = halves_sum(acc[i][0]);
+                    dot[i][1] = halves_sum(acc[i][1]);
+                }
+            };
+            if (my_rows > 4) dots(IntC<8>());
+            else if (my_rows > 2) dots(IntC<4>());
+            else if (my_rows > 0) dots(IntC<2>());
+        }
+        float prob[TOGETHER ? RPW : 1][2];
 #pragma unroll
         for (int i = 0; i < RPW; ++i) {
+            if constexpr (TOGETHER) prob[i][0] = prob[i][1] = 0.f;
             int r = warp + i * WARPS;
             if (r >= n_rows) continue;       // uniform within the warp
             int pos = DECODE ? first_pos : first_pos + r;
@@ -264,13 +321,17 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
                 r1 = p.dist_r1[head];
                 r2 = p.dist_r2[head];
             }
-            const float* qr = Qs + r * DH;
-            const float* k0 = Ks + lane * (DH + 1);
-            const float* k1 = Ks + (lane + 32) * (DH + 1);
-            // four partial sums a key: eight independent chains, so that a product does not wait for the one before it
-            // (with one chain a key the warp spent most cycles on the latency of its own additions)
-            float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
-            {
+            float s0, s1;
+            if constexpr (TOGETHER) {
+                s0 = dot[i][0];
+                s1 = dot[i][1];
+            } else {
+                const float* qr = Qs + r * DH;
+                const float* k0 = Ks + lane * KP;
+                const float* k1 = Ks + (lane + 32) * KP;
+                // four partial sums a key: eight independent chains, so that a product does not wait for the one before it
+                // (with one chain a key the warp spent most cycles on the latency of its own additions)
+                float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
                 int d = 0;
 #pragma unroll 4
                 for (; d + 4 <= DH; d += 4) {
@@ -285,8 +346,9 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
                     a0[0] = fmaf(qr[d], k0[d], a0[0]);
                     a1[0] = fmaf(qr[d], k1[d], a1[0]);
                 }
+                s0 = (a0[0] + a0[1]) + (a0[2] + a0[3]);
+                s1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
             }
-            float s0 = (a0[0] + a0[1]) + (a0[2] + a0[3]), s1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
             int kp0 = tile * LLB_PAGE + lane, kp1 = kp0 + 32;
             bool v0 = (kp0 >= lo || kp0 < keep) && kp0 <= pos, v1 = (kp1 >= lo || kp1 < keep) && kp1 <= pos;
             if (pooled) {
@@ -311,22 +373,58 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             float p0 = v0 ? expf(s0 - m_new) : 0.f, p1 = v1 ? expf(s1 - m_new) : 0.f;
             l[i] = l[i] * alpha + warp_sum(p0 + p1);
             m[i] = m_new;
-            float* ps = Ps + warp * LLB_PAGE;
-            __syncwarp();
-            ps[lane] = p0;
-            ps[lane + 32] = p1;
-            __syncwarp();
-            // keys outside, the lane's output dimensions inside: DPL independent chains
 #pragma unroll
             for (int e = 0; e < DPL; ++e) o[i][e] *= alpha;
+            if constexpr (TOGETHER) {
+                prob[i][0] = p0;
+                prob[i][1] = p1;
+            } else {
+                __syncwarp();
+                ps[lane] = p0;
+                ps[lane + 32] = p1;
+                __syncwarp();
+                // keys outside, the lane's output dimensions inside: DPL independent chains
 #pragma unroll 4
-            for (int j = 0; j < LLB_PAGE; ++j) {
-                const float pj = ps[j];
-                const float* vr = Vs + j * vs_stride + lane;
+                for (int j = 0; j < LLB_PAGE; ++j) {
+                    const float pj = ps[j];
+                    const float* vr = Vs + j * vs_stride + lane;
 #pragma unroll
-                for (int e = 0; e < DPL; ++e)
-                    if (lane + e * 32 < DV) o[i][e] = fmaf(pj, vr[e * 32], o[i][e]);
+                    for (int e = 0; e < DPL; ++e)
+                        if (lane + e * 32 < DV) o[i][e] = fmaf(pj, vr[e * 32], o[i][e]);
+                }
             }
+        }
+        if constexpr (TOGETHER) {
+            // all rows' probabilities of a key side by side, then a value at a time into all rows
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < RPW; i += 4)
+                    *reinterpret_cast<float4*>(ps + (lane + 32 * h) * PS + i) = make_float4(prob[i][h], prob[i + 1][h], prob[i + 2][h], prob[i + 3][h]);
+            __syncwarp();
+            auto sums = [&](auto rows) {
+                constexpr int N = decltype(rows)::value;
+#pragma unroll 4
+                for (int j = 0; j < LLB_PAGE; ++j) {
+                    float v[DPL], pj[N];
+#pragma unroll
+                    for (int e = 0; e < DPL; e += VW) {
+                        const float* src = Vs + j * vs_stride + out_dim(lane, e);
+                        if constexpr (VW == 4) *reinterpret_cast<float4*>(v + e) = *reinterpret_cast<const float4*>(src);
+                        else if constexpr (VW == 2) *reinterpret_cast<float2*>(v + e) = *reinterpret_cast<const float2*>(src);
+                        else v[e] = *src;
+                    }
+#pragma unroll
+                    for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(pj + i) = *reinterpret_cast<const float4*>(ps + j * PS + i);
+#pragma unroll
+                    for (int i = 0; i < N; ++i)
+#pragma unroll
+                        for (int e = 0; e < DPL; ++e) o[i][e] = fmaf(pj[i], v[e], o[i][e]);
+                }
+            };
+            if (my_rows > 4) sums(IntC<8>());
+            else if (my_rows > 0) sums(IntC<4>());
         }
     }
 
@@ -341,7 +439,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             float inv = 1.0f / l[i];
 #pragma unroll
             for (int e = 0; e < DPL; ++e) {
-                int d = lane + e * 32;
+                int d = out_dim(lane, e);
                 if (d < DV) {
                     if (p.out_f32) ((float*)p.out)[at + d] = o[i][e] * inv;
                     else ((T*)p.out)[at + d] = from_f32<T>(o[i][e] * inv);
@@ -351,7 +449,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             size_t slot = ((size_t)b * p.nh + head) * p.n_splits + blockIdx.x;
 #pragma unroll
             for (int e = 0; e < DPL; ++e) {
-                int d = lane + e * 32;
+                int d = out_dim(lane, e);
                 if (d < DV) p.part_o[slot * DV + d] = o[i][e];
             }
             if (lane == 0) {
@@ -389,7 +487,7 @@ __global__ void attn_combine_kernel(T* __restrict__ out, const float* __restrict
 }
 
 static size_t attn_smem_bytes(bool v_in_k) {
-    return (size_t)(ROWS * DH + LLB_PAGE * (DH + 1) + (v_in_k ? 0 : LLB_PAGE * DV) + WARPS * LLB_PAGE) * sizeof(float);
+    return (size_t)(ROWS * DH + LLB_PAGE * KP + (v_in_k ? 0 : LLB_PAGE * DV) + WARPS * LLB_PAGE * PS) * sizeof(float);
 }
 
 template <typename T, bool DECODE>

@@ -315,8 +315,14 @@ static int launch_f32(const float* X, const float* W, const void* bias, int bias
                       int ldx, int ldy, int splits, cudaStream_t stream) {
     auto kernel = gemm_f32_kernel<ROWS, TM>;
     constexpr int SMEM = F_STAGES * (ROWS + F_BN) * F_PITCH * (int)sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return -2000 - (int)e;
+    static bool configured[64] = {};          // function attributes belong to a device's copy of the kernel
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return -2000 - (int)e;
+        configured[dev] = true;
+    }
     const int m_tiles = (M + ROWS - 1) / ROWS, blocks = (K + F_BK - 1) / F_BK;
     const long long tiles = (long long)m_tiles * ((N + F_BN - 1) / F_BN);
     if (tiles > 2147483647ll) return (int)cudaErrorInvalidValue;

@@ -644,8 +644,14 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, int chunk, 
 template <bool STAGED, typename... A>
 static int launch_sample(int R, size_t smem, cudaStream_t stream, A... args) {
     auto kernel = sample_kernel<STAGED>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGED ? SMEM_MAX : (int)smem);
-    if (e != cudaSuccess) return -2000 - (int)e;
+    static bool configured[64] = {};          // function attributes belong to a device's copy of the kernel
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGED ? SMEM_MAX : (int)smem);
+        if (e != cudaSuccess) return -2000 - (int)e;
+        configured[dev] = true;
+    }
     llb_prefer_max_shared((const void*)kernel);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)R * SC);
