@@ -34,9 +34,11 @@ class StepContext:
         self.err, self.sm_count = err, sm_count
         B, T = n_seqs, n_tokens
         sizes = [T, T, T, B + 1, B, B, n_out] + [B * w for w in self.widths]
-        self._offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
-        self.meta = torch.empty(int(self._offs[-1]), dtype=torch.int32, device=self.device)
-        cut = [self.meta[self._offs[i]:self._offs[i + 1]] for i in range(len(sizes))]
+        self._offs = [0]
+        for n in sizes:
+            self._offs.append(self._offs[-1] + n)
+        self.meta = torch.empty(self._offs[-1], dtype=torch.int32, device=self.device)
+        cut = self.meta.split(sizes)
         (self.tokens, self.tok_seq, self.tok_pos, self.seq_start, self.seq_len_before, self.seq_slot,
          self.out_rows) = cut[:7]
         self._tables: Dict[int, torch.Tensor] = {g: cut[7 + g].view(B, w) for g, w in enumerate(self.widths)}
@@ -89,6 +91,10 @@ class StepContext:
 
     def kv(self, call: int) -> KVView:
         return self.cache.view(call, self._tables)
+
+    def kv_place(self, call: int):
+        """kv() as facts and addresses; see PagedCache.place."""
+        return self.cache.place(call, self._tables)
 
     def token_state(self) -> torch.Tensor:
         """int32 [n_slots, k] that the embedding part carries from step to step; row seq_slot[b] belongs to sequence b."""

@@ -4,6 +4,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import diagnostics
@@ -135,6 +136,16 @@ class Engine:
             raise StepError("feed() takes one token for every sequence of the step before it")
         kernels.scatter_i32(self.fed_tokens, ctx.seq_slot, tokens)
 
+    @staticmethod
+    def _ids(tokens) -> np.ndarray:
+        """A prompt's token ids as whole numbers, int(t) of each (what is beyond 62 bits is outside every vocabulary)."""
+        if type(tokens) is list and type(tokens[0]) is int:
+            try:
+                return np.array(tokens, dtype=np.int64)
+            except (OverflowError, TypeError, ValueError):
+                pass
+        return np.array([max(-1 << 62, min(int(t), 1 << 62)) for t in tokens], dtype=np.int64)
+
     def _forward(self, ctx, fed: bool):
         if fed:
             from .. import kernels
@@ -159,15 +170,19 @@ class Engine:
             raise StepError("a step that takes its tokens from the device brings one token per sequence")
         tokens, out_rows, base = [], [], 0
         for e, n in zip(entries, n_new):
-            for t in e.tokens:
-                if not fed and not (0 <= int(t) < self.spec.vocab_size):
-                    raise StepError(f"token id {t} is outside the vocabulary (0..{self.spec.vocab_size - 1})")
+            ids = self._ids(e.tokens) if n > 16 else [int(t) for t in e.tokens]
+            if not fed:
+                for t in ids if n <= 16 else ids[(ids < 0) | (ids >= self.spec.vocab_size)][:1].tolist():
+                    if not (0 <= t < self.spec.vocab_size):
+                        raise StepError(f"token id {t} is outside the vocabulary (0..{self.spec.vocab_size - 1})")
             for w in e.want:
                 if not (0 <= int(w) < n):
                     raise StepError(f"wanted index {w} is outside the {n} tokens of slot {e.slot}")
-            tokens += [int(t) for t in e.tokens]
+            tokens.append(ids)
             out_rows += [base + int(w) for w in e.want]
             base += n
+        # (a decode step's tokens stay a list, which is quicker for a few)
+        tokens = [t for ids in tokens for t in ids] if max(n_new) <= 16 else np.concatenate(tokens)
         book = self.cache.book
         if diagnostics.BOUNDS:
             wrong = book.audit()

@@ -6,10 +6,15 @@ from typing import Dict, List, Optional
 import torch
 
 from ..config.spec import ModelSpec
+from ..diagnostics import timers
+from ..kernels.ops import _check as check_launch
+from ..kernels.replay import Record
 from ..parts.base import BuildEnv, KVNeed, Part, SubLayer, TensorDecl, build_part, part_class
 
 
 class DecoderModel:
+    REPEAT_TOKENS = 4096          # steps of up to so many tokens repeat layers' launches from a record
+
     def __init__(self, spec: ModelSpec, env: BuildEnv):
         self.spec, self.env = spec, env
         self.embedding = build_part("embedding", spec.embedding, env)
@@ -151,10 +156,31 @@ class DecoderModel:
         residual = self.embedding.forward(ctx)
         pending = None
         first = self.reentry.remember(residual) if self.reentry is not None else None
+        record, known = None, None               # the layer taken down last, and its facts
         for c, call in enumerate(self.spec.order):
             if call.opens_pass is not None:
                 residual, pending = self.reentry.forward(residual, pending, first, call.opens_pass)
-            residual, pending = self.blocks[call.layer].forward(residual, pending, ctx, self.call_users[c])
+            block, users, facts = self.blocks[call.layer], self.call_users[c], None
+            # (taking a layer down costs a quarter of what repeating one saves: not for the last two.  A record holds its layer's
+            # buffers until the pass is over, which many tokens have no use for: their launches wait for the device)
+            if (record is not None or c + 2 < len(self.spec.order)) and residual.shape[0] <= self.REPEAT_TOKENS and not timers.enabled:
+                facts = block.repeat_facts(residual, pending, ctx, users) if hasattr(block, "repeat_facts") else None
+            if facts is None:
+                residual, pending = block.forward(residual, pending, ctx, users)
+                continue
+            if record is not None and known == facts[0] and record.delta is pending:
+                record.run(facts[1], check_launch)          # a layer like one taken down: its launches with this one's addresses
+                continue
+            taking, record = Record(), None
+            with taking:
+                after, left = block.forward(residual, pending, ctx, users)
+            # layers that leave the stream and a delta of the kind they found can follow one another; the delta of a repeated
+            # layer is left where the one taken down left its own
+            if after is residual and (left is None) == (pending is None) and (left is None or left.shape == pending.shape):
+                if taking.bind(facts[1]) and (left is None or taking.replace(pending.data_ptr(), left.data_ptr())):
+                    taking.delta = left                     # what a repeated layer finds pending, and leaves
+                    record, known = taking, facts[0]
+            residual, pending = after, left
         if ctx.out_rows.numel() == 0:
             return None
         from ..parts.block import settle

@@ -3,7 +3,7 @@ from __future__ import annotations
 import torch
 
 from .. import kernels
-from .base import KVNeed, Mixer, TensorDecl, build_part, register_part
+from .base import KVNeed, Mixer, TensorDecl, build_part, register_part, tensor_facts
 
 
 def decode_splits(ctx, n_kv_heads: int, clusters16: int = 0) -> int:
@@ -113,6 +113,22 @@ class GQAttention(Mixer):
             return False
         kernels.linear_into(self._attend(x, ctx, call), self.w_o, self.b_o, residual)
         return True
+
+    def repeat_facts(self, ctx, call):
+        """(facts, addresses): parts with equal facts launch the same kernels in a step, with these addresses in each other's
+        places.  None where that cannot be said."""
+        if type(self) is not GQAttention:
+            return None
+        tables = self.position.rotation_tables(ctx.max_position + 1) if self.position is not None else None
+        if self.position is not None and tables is None:
+            return None
+        kv = ctx.kv_place(call)
+        if kv is None:
+            return None
+        own = (self.w_qkv, self.b_qkv, self.w_o, self.b_o)
+        return ((self.kind, self.nh, self.nkvh, self.dh, self.scale, self.window, kv[0],
+                 tables and (tables[0].data_ptr(), tables[1].data_ptr(), tables[0].shape), tuple(map(tensor_facts, own))),
+                (*(t is not None and t.data_ptr() for t in own), *kv[1:]))
 
     def _attend(self, x, ctx, call):
         """Projections, position encoding, cache append and attention: [T, nh * dh], before the output projection."""

@@ -52,6 +52,11 @@ def part_class(category: str, kind: str) -> type:
     return cls
 
 
+def tensor_facts(t):
+    """What a launch can depend on in a tensor besides its contents."""
+    return None if t is None else (t.shape, t.dtype, t.is_contiguous(), t.data_ptr() & 15)
+
+
 def build_part(category: str, spec: PartSpec, env: "BuildEnv"):
     return part_class(category, spec.kind)(spec, env)
 

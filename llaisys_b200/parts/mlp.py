@@ -3,7 +3,7 @@ from __future__ import annotations
 import torch
 
 from .. import kernels
-from .base import FeedForward, TensorDecl, register_part
+from .base import FeedForward, TensorDecl, register_part, tensor_facts
 
 
 @register_part("ffn", "swiglu_mlp")
@@ -32,6 +32,13 @@ class SwiGLUMLP(FeedForward):
 
     def forward(self, x, ctx):
         return kernels.linear(kernels.linear_swiglu(x, self.gate_up), self.down)
+
+    def repeat_facts(self, ctx):
+        """See GQAttention.repeat_facts."""
+        if type(self) is not SwiGLUMLP:
+            return None
+        own = (self.gate_up, self.down)
+        return (self.kind, tuple(map(tensor_facts, own))), tuple(t.data_ptr() for t in own)
 
     def forward_into(self, x, ctx, residual):
         # a few tokens (decode): the three matrices stream through one launch that ends in the residual add

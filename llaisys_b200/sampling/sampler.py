@@ -50,9 +50,9 @@ class Sampler:
         p = self.params
         if p.greedy:
             return kernels.argmax(logits)
-        k = torch.tensor(list(keys), dtype=torch.int32).to(logits.device, non_blocking=True)
-        s = torch.tensor(list(steps), dtype=torch.int32).to(logits.device, non_blocking=True)
-        return kernels.sample(logits, p.temperature, p.top_k, p.top_p, self.seed, k, s)
+        keys, steps = list(keys), list(steps)
+        both = torch.tensor(keys + steps, dtype=torch.int32).to(logits.device, non_blocking=True)     # (one copy, not two)
+        return kernels.sample(logits, p.temperature, p.top_k, p.top_p, self.seed, both[:len(keys)], both[len(keys):])
 
     def __call__(self, logits: torch.Tensor, keys: Sequence[int], steps: Sequence[int]) -> List[int]:
         return self.on_device(logits, keys, steps).tolist()

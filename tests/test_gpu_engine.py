@@ -187,6 +187,37 @@ def test_captured_decode_steps_equal_uncaptured_ones(model, dtype):
             assert np.abs(row - outs[0][key]).max() < bound, key
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lengths", [[150, 9, 70], [300], [3, 2, 6]])
+def test_layers_that_are_repeated_from_a_record_equal_layers_that_run(model, dtype, lengths, monkeypatch):
+    """Six layers, so that layers are taken down and repeated (in configuration B behind a layer of another kind), prompts and
+    single tokens: the same numbers as with every layer run from Python, up to the order in which bfloat16's split sums
+    arrive (float32: the same launches, the same bits)."""
+    from llaisys_b200.kernels import replay
+    from llaisys_b200.parts.block import PreNormResidual
+    cfg = dict(CONFIGS[model.name], num_hidden_layers=6)
+    folder = make_folder(model._tmp / f"six{GAIN[dtype]}", cfg, seed=ord(model.name), attn_gain=GAIN[dtype])
+    reqs = random_requests(cfg, [n + 6 for n in lengths], seed=23)
+    ran, run = [], replay.Record.run
+
+    def counted(self, *args):
+        ran.append(1)
+        run(self, *args)
+
+    monkeypatch.setattr(replay.Record, "run", counted)
+    outs = []
+    for repeat in (True, False):
+        if not repeat:
+            monkeypatch.setattr(PreNormResidual, "repeat_facts", lambda self, *a: None)
+        engine = build_engine(folder, dtype, max_tokens=64 * 8, use_graphs=False)
+        outs.append(run_batches(engine, reqs, [list(range(len(reqs)))], list(lengths)))
+        assert bool(ran) == repeat
+        ran.clear()
+    rms = np.sqrt(np.mean([np.mean(r ** 2) for r in outs[1].values()]))
+    for key, row in outs[1].items():
+        assert np.abs(row - outs[0][key]).max() <= (0 if dtype == torch.float32 else 0.05 * rms), key
+
+
 def test_padding_and_company_change_nothing(model):
     """float32: a request's logits are the same alone and in a batch, up to rounding."""
     name, folder, oracle, requests = model
