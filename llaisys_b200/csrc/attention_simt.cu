@@ -229,6 +229,15 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
                            : page + (size_t)j * page_row + d;
             };
             if (WIDTH % VEC == 0 && (((uintptr_t)pool | (uintptr_t)fresh) & 15) == 0 && kv_stride % VEC == 0) {
+                if (sizeof(T) == 4 && pitch % 4 == 0) {          // nothing to convert: all of a thread's pieces go their own way
+                    for (int i = tid; i < PIECES; i += WARPS * 32) {
+                        const int j = i / PER, d = (i - j * PER) * VEC;
+                        const T* src = source(j, d);
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + j * pitch + d)),
+                                     "l"(src ? src : page ? page : fresh), "r"(src ? 16 : 0) : "memory");
+                    }
+                    return;
+                }
                 for (int i0 = tid; i0 < PIECES; i0 += BATCH * WARPS * 32) {
                     uint4 raw[BATCH];
 #pragma unroll
@@ -265,6 +274,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             if (!p.v_in_k)
                 fetch_tile(IntC<DV>(), Vs, DV, vpool, cached ? vpool + paged_row(table, p.ring, p0, vh, cache_heads, DV, p.pinned) : nullptr, DV,
                            vnew, vh * DV);
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
         __syncthreads();
         const int my_rows = n_rows > warp ? (n_rows - warp + WARPS - 1) / WARPS : 0;      // rows warp, warp + WARPS, ... of the block
@@ -303,29 +313,78 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
             else if (my_rows > 2) dots(IntC<4>());
             else if (my_rows > 0) dots(IntC<2>());
         }
-        float prob[TOGETHER ? RPW : 1][2];
-#pragma unroll
-        for (int i = 0; i < RPW; ++i) {
-            if constexpr (TOGETHER) prob[i][0] = prob[i][1] = 0.f;
-            int r = warp + i * WARPS;
-            if (r >= n_rows) continue;       // uniform within the warp
+        // a row's scaled, capped and masked scores from its dot products (-inf: not seen), and which of the two are seen
+        auto masked = [&](int r, float& s0, float& s1, bool& v0, bool& v1) {
             int pos = DECODE ? first_pos : first_pos + r;
             int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
             if (p.chunk > 0) lo = max(lo, (pos / p.chunk) * p.chunk);
-            const int blocks_seen = pooled ? max(0, (pos - p.window + 1) / p.pool) : 0;
             float row_scale = p.scale;
             if (p.q_temp_every > 0) row_scale *= 1.0f + p.q_temp_coef * logf((float)((pos + 1) / p.q_temp_every + 1));
-            float r1 = 0.f, r2 = 0.f;
-            if (p.dist_r1) {
-                const int head = row_head0 + (DECODE ? r : 0);
-                r1 = p.dist_r1[head];
-                r2 = p.dist_r2[head];
+            int kp0 = tile * LLB_PAGE + lane, kp1 = kp0 + 32;
+            v0 = (kp0 >= lo || kp0 < keep) && kp0 <= pos, v1 = (kp1 >= lo || kp1 < keep) && kp1 <= pos;
+            if (pooled) {
+                const int blocks_seen = max(0, (pos - p.window + 1) / p.pool);
+                v0 = kp0 < blocks_seen;
+                v1 = kp1 < blocks_seen;
             }
-            float s0, s1;
-            if constexpr (TOGETHER) {
-                s0 = dot[i][0];
-                s1 = dot[i][1];
-            } else {
+            s0 *= row_scale;
+            s1 *= row_scale;
+            if (p.softcap > 0.f) {
+                s0 = p.softcap * tanhf(s0 / p.softcap);
+                s1 = p.softcap * tanhf(s1 / p.softcap);
+            }
+            s0 = v0 ? s0 : -INFINITY;
+            s1 = v1 ? s1 : -INFINITY;
+            if (p.dist_r1 && !pooled) {
+                const int head = row_head0 + (DECODE ? r : 0);
+                const float r1 = p.dist_r1[head], r2 = p.dist_r2[head];
+                if (v0) s0 -= r1 * log1pf(r2 * (float)(pos - kp0));
+                if (v1) s1 -= r1 * log1pf(r2 * (float)(pos - kp1));
+            }
+        };
+        float prob[TOGETHER ? RPW : 1][2];
+        if constexpr (TOGETHER) {
+            // every step for all rows before the next: a row's shuffles wait for one another, the rows' do not
+            float top[RPW], sum[RPW];
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) {
+                bool v0, v1;
+                prob[i][0] = prob[i][1] = top[i] = -INFINITY;
+                if (i >= my_rows) continue;                        // uniform within the warp
+                float s0 = dot[i][0], s1 = dot[i][1];
+                masked(warp + i * WARPS, s0, s1, v0, v1);
+                prob[i][0] = s0;
+                prob[i][1] = s1;
+                top[i] = fmaxf(s0, s1);
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int i = 0; i < RPW; ++i) top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], off));
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) {
+                const float m_new = fmaxf(m[i], top[i]);
+                const bool any = m_new != -INFINITY;               // no visible key yet: nothing changes
+                const float alpha = any ? expf(m[i] - m_new) : 1.f;        // exp(-inf) = 0 on the first visible tile
+#pragma unroll
+                for (int h = 0; h < 2; ++h) prob[i][h] = any ? expf(prob[i][h] - m_new) : 0.f;       // (unseen: exp(-inf))
+                sum[i] = prob[i][0] + prob[i][1];
+                l[i] *= alpha;
+                m[i] = m_new;
+#pragma unroll
+                for (int e = 0; e < DPL; ++e) o[i][e] *= alpha;
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int i = 0; i < RPW; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], off);
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) l[i] += sum[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) {
+                int r = warp + i * WARPS;
+                if (r >= n_rows) continue;       // uniform within the warp
                 const float* qr = Qs + r * DH;
                 const float* k0 = Ks + lane * KP;
                 const float* k1 = Ks + (lane + 32) * KP;
@@ -346,44 +405,22 @@ __global__ void __launch_bounds__(WARPS * 32) attn_kernel(AttnParams p) {
                     a0[0] = fmaf(qr[d], k0[d], a0[0]);
                     a1[0] = fmaf(qr[d], k1[d], a1[0]);
                 }
-                s0 = (a0[0] + a0[1]) + (a0[2] + a0[3]);
-                s1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
-            }
-            int kp0 = tile * LLB_PAGE + lane, kp1 = kp0 + 32;
-            bool v0 = (kp0 >= lo || kp0 < keep) && kp0 <= pos, v1 = (kp1 >= lo || kp1 < keep) && kp1 <= pos;
-            if (pooled) {
-                v0 = kp0 < blocks_seen;
-                v1 = kp1 < blocks_seen;
-            }
-            s0 *= row_scale;
-            s1 *= row_scale;
-            if (p.softcap > 0.f) {
-                s0 = p.softcap * tanhf(s0 / p.softcap);
-                s1 = p.softcap * tanhf(s1 / p.softcap);
-            }
-            s0 = v0 ? s0 : -INFINITY;
-            s1 = v1 ? s1 : -INFINITY;
-            if (p.dist_r1 && !pooled) {
-                if (v0) s0 -= r1 * log1pf(r2 * (float)(pos - kp0));
-                if (v1) s1 -= r1 * log1pf(r2 * (float)(pos - kp1));
-            }
-            float m_new = fmaxf(m[i], warp_max(fmaxf(s0, s1)));
-            if (m_new == -INFINITY) continue;          // no visible key yet (uniform)
-            float alpha = expf(m[i] - m_new);           // exp(-inf) = 0 on the first visible tile
-            float p0 = v0 ? expf(s0 - m_new) : 0.f, p1 = v1 ? expf(s1 - m_new) : 0.f;
-            l[i] = l[i] * alpha + warp_sum(p0 + p1);
-            m[i] = m_new;
-#pragma unroll
-            for (int e = 0; e < DPL; ++e) o[i][e] *= alpha;
-            if constexpr (TOGETHER) {
-                prob[i][0] = p0;
-                prob[i][1] = p1;
-            } else {
+                float s0 = (a0[0] + a0[1]) + (a0[2] + a0[3]), s1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
+                bool v0, v1;
+                masked(r, s0, s1, v0, v1);
+                float m_new = fmaxf(m[i], warp_max(fmaxf(s0, s1)));
+                if (m_new == -INFINITY) continue;          // no visible key yet (uniform)
+                float alpha = expf(m[i] - m_new);           // exp(-inf) = 0 on the first visible tile
+                float p0 = v0 ? expf(s0 - m_new) : 0.f, p1 = v1 ? expf(s1 - m_new) : 0.f;
+                l[i] = l[i] * alpha + warp_sum(p0 + p1);
+                m[i] = m_new;
                 __syncwarp();
                 ps[lane] = p0;
                 ps[lane + 32] = p1;
                 __syncwarp();
                 // keys outside, the lane's output dimensions inside: DPL independent chains
+#pragma unroll
+                for (int e = 0; e < DPL; ++e) o[i][e] *= alpha;
 #pragma unroll 4
                 for (int j = 0; j < LLB_PAGE; ++j) {
                     const float pj = ps[j];

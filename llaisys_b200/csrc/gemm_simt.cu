@@ -191,18 +191,21 @@ gemm_rows_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, c
 }
 
 // More rows: bound by the FMA units.  A block computes ROWS x 128 outputs from a ring of three k-blocks of 32 (cp.async, 16-byte
-// pieces, rows 144 bytes apart so that eight neighbouring rows are read without bank conflicts); a thread has TM x 8
-// outputs (16 TM FMAs for every TM + 8 loads of 16 bytes).  With ROWS = 64, two blocks of four warps share an SM; rows of 16
-// and 32 are for products that would leave most of a tile empty (41 and 56 us for 16 and 32 rows against 17,920 x 1,536, 95 with 64).
-// At 46 TFLOP/s (256 x 151,936 x 1,536) shared-memory reads, a byte an FMA, take as long as the FMAs.  (4-byte loads, a
-// transposing store and 4 x 4 outputs a thread before: 13 TFLOP/s; a 256-token step of the 1.5B shape 59 -> 24 ms.)
+// pieces, rows 144 bytes apart so that eight neighbouring rows are read without bank conflicts); a thread has TM x TN
+// outputs (4 TM TN FMAs for every TM + TN loads of 16 bytes).  With ROWS = 64, two blocks of four warps share an SM; rows of 16
+// and 32 are for products that would leave most of a tile empty: 34 and 52 us for 16 and 32 rows against 17,920 x 1,536, 91 for 64;
+// 233, 387 and 700 against 151,936 x 1,536.  (2 x 8 and 4 x 8 outputs a thread for 16 and 32 rows: 41 and 53, 295 and 394.)
+// 256 rows reach 46 TFLOP/s (151,936 x 1,536), of 74 that chains of such FMAs alone reach: the FMA pipe is 60 % busy, two warps a
+// scheduler cover neither their reads of shared memory nor their barriers.  Four warps with 8 x 4 outputs (45), 4 x 8 (43),
+// and reads two k ahead in registers (46) were no faster.  (4-byte loads, a transposing store and 4 x 4 outputs a thread
+// before: 13 TFLOP/s; a 256-token step of the 1.5B shape 59 -> 21 ms with this and the attention's changes.)
 // gridDim.z > 1: K is cut into ranges, each range's partial product goes to its plane of `part`, and gemm_planes_f32_kernel adds them.
 constexpr int F_BN = 128, F_BK = 32, F_PITCH = F_BK + 4, F_STAGES = 3;
-template <int ROWS, int TM>
-__global__ void __launch_bounds__(ROWS / TM * 16, ROWS >= 64 ? 2 : 3)
+template <int ROWS, int TM, int TN>
+__global__ void __launch_bounds__(ROWS / TM * (F_BN / TN), ROWS >= 64 ? 2 : 3)
 gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const void* __restrict__ bias, int bias_dtype,
                 float* __restrict__ Y, float* __restrict__ part, int M, int N, int K, int ldx, int ldy, int m_tiles, int k_range) {
-    constexpr int THREADS = ROWS / TM * 16, TN = 8;
+    constexpr int THREADS = ROWS / TM * (F_BN / TN), WN = F_BN / (8 * TN);      // (warps side by side)
     constexpr int STAGE = (ROWS + F_BN) * F_PITCH;                     // floats
     extern __shared__ __align__(16) float ring[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -224,8 +227,8 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const 
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
         }
     };
-    // a warp's outputs: 4 TM rows x 64 columns; lane (ly, lx) has rows ly + 4 i and columns lx + 8 j of them
-    const int lx = lane & 7, ly = lane >> 3, wn = warp & 1, wm = warp >> 1;
+    // a warp's outputs: 4 TM rows x 8 TN columns; lane (ly, lx) has rows ly + 4 i and columns lx + 8 j of them
+    const int lx = lane & 7, ly = lane >> 3, wn = warp % WN, wm = warp / WN;
     f32x2 acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
@@ -242,7 +245,7 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const 
         if (kb + F_STAGES - 1 < n_blocks) fetch(kb + F_STAGES - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* xs = ring + (kb % F_STAGES) * STAGE + (wm * 4 * TM + ly) * F_PITCH;
-        const float* ws = ring + (kb % F_STAGES) * STAGE + (ROWS + wn * 64 + lx) * F_PITCH;
+        const float* ws = ring + (kb % F_STAGES) * STAGE + (ROWS + wn * 8 * TN + lx) * F_PITCH;
 #pragma unroll
         for (int k = 0; k < F_BK; k += 4) {
             ulonglong2 b[TN];
@@ -268,7 +271,7 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const 
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int n = n0 + wn * 64 + lx + 8 * j;
+            const int n = n0 + wn * 8 * TN + lx + 8 * j;
             if (n >= N) continue;
             float v = halves_sum(acc[i][j]);
             if (bias && !planes) v += bias_at(bias, bias_dtype, n);
@@ -277,17 +280,33 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, const 
     }
 }
 
-// Y = sum of the planes, in their order, + bias
+// Y = sum of the planes, in their order, + bias; VEC neighbouring columns a thread (4: N and ldy multiples of 4, aligned Y)
+template <int VEC>
 __global__ void __launch_bounds__(256)
 gemm_planes_f32_kernel(const float* __restrict__ part, int planes, const void* __restrict__ bias, int bias_dtype, float* __restrict__ Y,
                        int M, int N, int ldy) {
     llb_grid_dependency_sync();
-    const size_t n_all = (size_t)M * N;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n_all; i += (size_t)gridDim.x * 256) {
-        float s = part[i];
-        for (int q = 1; q < planes; ++q) s += part[q * n_all + i];
-        const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
-        Y[(size_t)m * ldy + n] = bias ? s + bias_at(bias, bias_dtype, n) : s;
+    const int n = (blockIdx.x * 256 + threadIdx.x) * VEC;
+    if (n >= N) return;
+    const size_t plane = (size_t)M * N;
+    for (int m = blockIdx.y; m < M; m += gridDim.y) {
+        const float* src = part + (size_t)m * N + n;
+        float s[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) s[e] = 0.f;
+#pragma unroll 4
+        for (int q = 0; q < planes; ++q) {
+            float v[VEC];
+            if constexpr (VEC == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src + q * plane);
+            else v[0] = src[q * plane];
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) s[e] += v[e];
+        }
+        if (bias)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) s[e] += bias_at(bias, bias_dtype, n + e);
+        if constexpr (VEC == 4) *reinterpret_cast<float4*>(Y + (size_t)m * ldy + n) = *reinterpret_cast<float4*>(s);
+        else Y[(size_t)m * ldy + n] = s[0];
     }
 }
 
@@ -310,10 +329,10 @@ static int f32_splits(int M, int N, int K, int sms) {
     return best;
 }
 
-template <int ROWS, int TM>
+template <int ROWS, int TM, int TN>
 static int launch_f32(const float* X, const float* W, const void* bias, int bias_dtype, float* Y, float* part, int M, int N, int K,
                       int ldx, int ldy, int splits, cudaStream_t stream) {
-    auto kernel = gemm_f32_kernel<ROWS, TM>;
+    auto kernel = gemm_f32_kernel<ROWS, TM, TN>;
     constexpr int SMEM = F_STAGES * (ROWS + F_BN) * F_PITCH * (int)sizeof(float);
     static bool configured[64] = {};          // function attributes belong to a device's copy of the kernel
     int dev = 0;
@@ -326,11 +345,14 @@ static int launch_f32(const float* X, const float* W, const void* bias, int bias
     const int m_tiles = (M + ROWS - 1) / ROWS, blocks = (K + F_BK - 1) / F_BK;
     const long long tiles = (long long)m_tiles * ((N + F_BN - 1) / F_BN);
     if (tiles > 2147483647ll) return (int)cudaErrorInvalidValue;
-    llb_launch(kernel, dim3((unsigned)tiles, 1, splits), dim3(ROWS / TM * 16), SMEM, stream, X, W, bias, bias_dtype, Y, part, M, N, K, ldx,
+    llb_launch(kernel, dim3((unsigned)tiles, 1, splits), dim3(ROWS / TM * (F_BN / TN)), SMEM, stream, X, W, bias, bias_dtype, Y, part, M, N, K, ldx,
                ldy, m_tiles, (blocks + splits - 1) / splits * F_BK);
-    if (splits > 1)
-        llb_launch(gemm_planes_f32_kernel, dim3((unsigned)min(((size_t)M * N + 255) / 256, (size_t)148 * 16)), dim3(256), 0, stream,
+    if (splits > 1) {
+        const bool vec = N % 4 == 0 && ldy % 4 == 0 && (((uintptr_t)Y | (uintptr_t)part) & 15) == 0;
+        const int columns = vec ? N / 4 : N;
+        llb_launch(vec ? gemm_planes_f32_kernel<4> : gemm_planes_f32_kernel<1>, dim3((columns + 255) / 256, M < 65535 ? M : 65535), dim3(256), 0, stream,
                    (const float*)part, splits, bias, bias_dtype, Y, M, N, ldy);
+    }
     return llb_status();
 }
 
@@ -382,9 +404,9 @@ LLB_API int llb_gemm_simt(const void* X, int x_dtype, const void* W, int w_dtype
         }
         int splits = f32_splits(M, N, K, sms);
         if (!part || part_elems < (long long)splits * M * N) splits = 1;
-        return M <= 16 ? launch_f32<16, 2>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream)
-             : M <= 32 ? launch_f32<32, 4>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream)
-                       : launch_f32<64, 8>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream);
+        return M <= 16 ? launch_f32<16, 4, 4>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream)
+             : M <= 32 ? launch_f32<32, 8, 4>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream)
+                       : launch_f32<64, 8, 8>(x, w, bias, bias_dtype, (float*)Y, part, M, N, K, ldx, ldy, splits, stream);
     }
     if ((N + 63) / 64 > 2147483647 || (M + 63) / 64 > 65535) return (int)cudaErrorInvalidValue;
     LLB_DISPATCH_DTYPE(x_dtype, TX, {
