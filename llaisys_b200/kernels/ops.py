@@ -1228,7 +1228,7 @@ def moe_gather_rows(x: torch.Tensor, plan: MoePlan) -> torch.Tensor:
     assert x.stride(1) == 1
     out = _new((plan.n_pairs, x.shape[1]), dtype=x.dtype, device=x.device)
     f = _fn(_moe_lib(), "llb_moe_gather_rows", [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p])
-    _check(f(_ptr(x), _dt(x), x.stride(0), _ptr(plan.pair_of), plan.top, _ptr(plan.n_tiles), _ptr(out), plan.n_pairs, x.shape[1], _stream()),
+    _check(f(_ptr(x), _dt(x), x.stride(0), _ptr(plan.slot_of), plan.top, _ptr(plan.n_tiles), _ptr(out), plan.n_pairs // plan.top, x.shape[1], _stream()),
            "experts' rows in slot order")
     return out
 

@@ -671,6 +671,30 @@ def test_feed_forward_in_one_launch(T, H, I, stages):
     assert float((two - res).abs().max()) <= 2.0 ** -7 * float((res - res0).abs().max()) + 1e-3
 
 
+@pytest.mark.parametrize("T,E,top,rows,outside", [(1, 1, 1, 16, 0), (8, 64, 6, 16, 0), (700, 33, 3, 64, 2), (2048, 64, 6, 256, 0),
+                                                  (5462, 40, 3, 64, 1), (6000, 200, 3, 16, 40)])
+def test_plan_groups_the_pairs(T, E, top, rows, outside):
+    """Every pair has a slot of its own, an expert's slots follow one another and are cut into tiles, pairs of experts beyond E come
+    last; up to 16,384 pairs (read once) and beyond (read twice).  The rows in slot order are the tokens'."""
+    from llaisys_b200 import kernels
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    idx = torch.rand(T, E + outside, device=DEV, generator=gen).topk(top, -1).indices.int()
+    plan = kernels.moe_plan(idx, E, rows)
+    pair, e = plan.pair_of.long(), idx.reshape(-1).clamp_max(E)
+    assert torch.equal(plan.slot_of.long()[pair], torch.arange(T * top, device=DEV))
+    got = e[pair]
+    assert bool((got[1:] >= got[:-1]).all())
+    count = torch.bincount(e, minlength=E + 1)[:E].tolist()
+    want, first = [], 0
+    for x, c in enumerate(count):
+        want += [(x, first + r, min(rows, c - r)) for r in range(0, c, rows)]
+        first += c
+    assert plan.n_tiles[:2].tolist() == [len(want), first]
+    assert list(zip(*plan.tiles.view(3, -1)[:, :len(want)].tolist())) == want
+    for x in (torch.randn(T, 24, device=DEV, generator=gen), torch.randn(T, 77, device=DEV, generator=gen).bfloat16()[:, 1:70]):
+        assert torch.equal(kernels.moe_gather_rows(x, plan)[:first], x[pair[:first] // top])
+
+
 @pytest.mark.parametrize("T,E,top,H,ff,skew", [(40, 1, 1, 64, 8, 1.0), (257, 1, 1, 72, 264, 1.0), (300, 2, 2, 128, 256, 1.0), (700, 5, 3, 200, 520, 3.0),
                                                (1500, 16, 2, 512, 136, 1.5), (512, 3, 1, 64, 1408, 9.0)])
 def test_experts_products_in_tiles_of_256_slots(T, E, top, H, ff, skew):
