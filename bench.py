@@ -365,7 +365,7 @@ def stamps_run(args, model, cfg, rng) -> int:
 
 def products_run(args, cfg) -> int:
     """The four matrix products of a layer timed alone at --tokens tokens, with every kernel that takes them:
-    the one-CTA tcgen05 kernel and, for more than 256 tokens, the paired-SM kernel (which the library chooses)."""
+    the one-CTA tcgen05 kernel and, for more than 128 tokens, the paired-SM kernel (which the library chooses)."""
     import torch
 
     from llaisys_b200.kernels import ops
@@ -403,7 +403,7 @@ def products_run(args, cfg) -> int:
         w = (torch.randn(N, K, device=dev) * 0.05).to(torch.bfloat16)
         run = (lambda plan: ops.linear_swiglu(x, w, plan=plan)) if dual else (lambda plan: ops.linear(x, w, None, plan=plan))
         plans = [("one CTA per tile", ops.tc_plan(T, N // 2 if dual else N, K, ops._sm_count(dev), dual))]
-        if T > 256:
+        if T > 128:
             plans.append(("paired SMs", ("pair",)))
         graphs = [(label, graph_of(lambda plan=plan: run(plan))) for label, plan in plans]
         # for scale only: the library's product of the same operands (cuBLAS through torch.matmul; for gate/up

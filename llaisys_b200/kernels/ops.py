@@ -563,7 +563,10 @@ def _gemm_tc_pair(x, weight, bias, out, dual_offset=0, glu=SWIGLU):
 def _gemm_tc(x, weight, bias, out, dual_offset=0, plan=None, glu=SWIGLU):
     M, K = x.shape
     N = weight.shape[0]
-    if plan is None and M > 256 and _pair_ok(out, dual_offset or N):
+    # Beyond 128 tokens on pairs of SMs: a tile of 256 tokens takes one SM as long as it takes a pair to do two of them.  One CTA a tile
+    # / paired, us: gate/up of 2 x 8,960 x 1,536 at 128 tokens 15.1 / 16.8, 130 tokens 21.6 / 16.8, 256 tokens 22.4 / 17.2; q/k/v of
+    # 4,608 x 3,584 17.1 / 20.6, 22.5 / 20.7, 23.1 / 21.2; gate/up of 2 x 18,944 x 3,584 44.0 / 49.6, 49.9 / 49.8, 54.5 / 53.2.
+    if plan is None and M > 128 and _pair_ok(out, dual_offset or N):
         plan = ("pair",)
     if plan is not None and plan[0] == "pair":
         return _gemm_tc_pair(x, weight, bias, out, dual_offset, glu)

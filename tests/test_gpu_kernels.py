@@ -464,6 +464,20 @@ def test_linear_swiglu_on_paired_sms_and_on_single_ones(T, I, K, plan):
     assert kernels.tc_error(DEV) == 0
 
 
+@pytest.mark.parametrize("T", [128, 129, 200, 256])
+@pytest.mark.parametrize("N,K", [(80, 200), (528, 1536), (272, 2112)])
+def test_products_around_the_first_paired_tile(T, N, K):
+    """From 129 tokens on the products with bfloat16 results run on pairs of SMs, the first 256 in one tile of which the second CTA's
+    half may hold a single token; both gate/up variants."""
+    from llaisys_b200 import kernels
+    x, w, b = _tc_case(T, N, K, T + N, bias=torch.bfloat16)
+    _close(kernels.linear(x, w, b), plain.linear(x.double().cpu().numpy(), w.double().cpu().numpy(), b.double().cpu().numpy()),
+           torch.bfloat16, atol=5e-3)
+    gu = plain.linear(x.double().cpu().numpy(), w.double().cpu().numpy())
+    _close(kernels.linear_swiglu(x, w), plain.swiglu(gu[:, :N // 2], gu[:, N // 2:]), torch.bfloat16, atol=5e-3)
+    assert kernels.tc_error(DEV) == 0
+
+
 @pytest.mark.parametrize("bn", [16, 32, 64, 128, 256])
 @pytest.mark.parametrize("splits,cluster", [(1, 0), (2, 0), (5, 0), (2, 1), (4, 1), (8, 1)])
 def test_linear_tensor_cores_every_tile_and_split(bn, splits, cluster):
